@@ -18,7 +18,11 @@
 // key order among equal maxima); A_h and kappa_h are constants of the support (rest areas,
 // masses and the stored barycentric coordinates). dE/dr is the gradient the reference's
 // direction refinement builds (intersection_resolver2.cpp:1268-1320).
+#include <cooperative_groups.h>
+
 #include "u26_internal.h"
+
+namespace cg = cooperative_groups;
 
 namespace u26
 {
@@ -129,98 +133,223 @@ namespace u26
 			atomicAdd(gx + 3 * size_t(v) + 2, g.z);
 		}
 
-		// One warp per contour: forward J, E (canonical 32-lane strided sums), then the
-		// vector-Jacobian products for the upstream gradients gJ, gE (when given).
-		__global__ void adjoint_kernel(const float* __restrict__ x, const u26_prp_hit* __restrict__ hits, const uint32_t* __restrict__ off,
-			uint32_t nc, const float* __restrict__ dirs, const float* __restrict__ va, const float* __restrict__ ea, const float* __restrict__ fa,
-			const float* __restrict__ vm, float* __restrict__ J_out, float* __restrict__ E_out, const float* __restrict__ gJ,
-			const float* __restrict__ gE, float* __restrict__ grad_dirs, float* __restrict__ grad_x)
+		// The deepest hit of some of a contour's hits: the deeper of two, the earlier of equals. A NaN
+		// depth never wins, except that of the contour's first hit, which stays.
+		struct Deepest
 		{
-			const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-			const int lane = threadIdx.x & 31;
-			if (c >= nc)
+			float depth;
+			uint32_t hit; // kInvalid: none
+		};
+		__device__ __forceinline__ void deepest(Deepest& a, float depth, uint32_t hit, uint32_t first)
+		{
+			if (hit == kInvalid || (isnan(a.depth) && a.hit == first))
 				return;
-			const uint32_t h0 = off[c], h1 = off[c + 1];
-			const f3 r = mk3(dirs[3 * c], dirs[3 * c + 1], dirs[3 * c + 2]);
-			float sA = 0.0f, sE = 0.0f, dmax = -INFINITY;
-			uint32_t imax = kInvalid;
-			for (uint32_t i = h0 + lane; i < h1; i += 32)
+			if (a.hit == kInvalid || depth > a.depth || (depth == a.depth && hit < a.hit) || (isnan(depth) ? hit == first : isnan(a.depth)))
 			{
-				const u26_prp_hit h = hits[i];
-				const HitGeo G = hit_geo(h, x, r);
-				sA = sA + hit_area(h, va, ea, fa);
-				const float kap = hit_kappa(h, vm);
-				const float sd = G.delta + 3e-3f;
-				sE = sE + (kap > 1e-8f ? (sd * sd) / kap : 0.0f);
-				if (G.delta > dmax || imax == kInvalid)
+				a.depth = depth;
+				a.hit = hit;
+			}
+		}
+
+		// A cluster of gridDim.x / nc blocks per contour: forward J, E, then the vector-Jacobian
+		// products for the upstream gradients gJ, gE (when given).
+		// A hit costs one 48-byte record, four gathered vertices and about 250 flops, so one warp
+		// walking a contour's hits is a chain of gather latencies (5 ms for 90,526 hits, and as much
+		// again for the gradients). Here the hits are spread over up to 8,192 threads (the rule
+		// is in u26_prp_adjoint); what stays serial is the canonical summation order of the areas
+		// and costs (32 lanes striding over the hits, then an xor butterfly): the terms go to shared
+		// memory, round by round, and two warps of the cluster add them up from there (distributed
+		// shared memory, one add per 32 hits). No scratch memory, and the results
+		// do not depend on timing, but for the order of grad_x's atomics. The gradients in the
+		// direction are summed in double, in a fixed order. Forward and backward of one contour of
+		// 90,526 hits: 9.1 ms with a warp per contour, 0.20 ms now (0.17 ms of it the host's calls).
+		template <int NT>
+		__global__ void __launch_bounds__(NT, 1024 / NT) adjoint_kernel(const float* __restrict__ x, const u26_prp_hit* __restrict__ hits,
+			const uint32_t* __restrict__ off, const float* __restrict__ dirs, const float* __restrict__ va, const float* __restrict__ ea,
+			const float* __restrict__ fa, const float* __restrict__ vm, float* __restrict__ J_out, float* __restrict__ E_out,
+			const float* __restrict__ gJ, const float* __restrict__ gE, float* __restrict__ grad_dirs, float* __restrict__ grad_x)
+		{
+			constexpr int kWarps = NT / 32;
+			constexpr uint32_t kSlice = 4 * NT; // a block's hits per round
+			__shared__ Deepest s_warp[kWarps];
+			__shared__ Deepest s_block;
+			__shared__ float s_area[kSlice], s_cost[kSlice];
+			__shared__ float s_sum[2];
+			__shared__ double s_gr[kWarps][3];
+			__shared__ double s_gr_block[3];
+			cg::cluster_group cluster = cg::this_cluster();
+			const uint32_t nb = cluster.num_blocks(), rank = cluster.block_rank();
+			const uint32_t c = blockIdx.x / nb;
+			const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+			const uint32_t h0 = off[c], h1 = off[c + 1];
+			const uint32_t n = h1 > h0 ? h1 - h0 : 0u, round = nb * kSlice;
+			const f3 r = mk3(dirs[3 * c], dirs[3 * c + 1], dirs[3 * c + 2]);
+			Deepest my = { -INFINITY, kInvalid };
+			float sum = 0.0f; // lanes of the summing warps: 0 the areas, 1 the costs
+			for (uint64_t q = 0; q < n; q += round)
+			{
+				const uint32_t left = uint32_t(min(uint64_t(round), n - q));
+#pragma unroll 1
+				for (uint32_t k = threadIdx.x; k < kSlice; k += NT)
 				{
-					dmax = G.delta;
-					imax = i;
+					if (rank * kSlice + k >= left)
+						break;
+					const uint32_t i = h0 + uint32_t(q) + rank * kSlice + k;
+					const u26_prp_hit h = hits[i];
+					const HitGeo G = hit_geo(h, x, r);
+					s_area[k] = hit_area(h, va, ea, fa);
+					const float kap = hit_kappa(h, vm);
+					const float sd = G.delta + 3e-3f;
+					s_cost[k] = kap > 1e-8f ? (sd * sd) / kap : 0.0f;
+					deepest(my, G.delta, i, h0);
 				}
+				cluster.sync();
+				if (rank == 0 && warp < 2)
+				{
+					// 32 loads in flight: a remote load's latency is about eight adds'
+					for (uint32_t b = 0; b < nb && b * kSlice < left; b++)
+					{
+						const float* p = cluster.map_shared_rank(warp == 0 ? s_area : s_cost, b);
+						const uint32_t m = min(kSlice, left - b * kSlice);
+						uint32_t k = lane;
+						for (; k - lane + 1024u <= m; k += 1024u)
+						{
+							float t[32];
+#pragma unroll
+							for (int u = 0; u < 32; u++)
+								t[u] = p[k + 32 * u];
+#pragma unroll
+							for (int u = 0; u < 32; u++)
+								sum = sum + t[u];
+						}
+						for (; k < m; k += 32u)
+							sum = sum + p[k];
+					}
+				}
+				cluster.sync(); // the terms are read before the next round's are written
 			}
 #pragma unroll
 			for (int o = 16; o >= 1; o >>= 1)
 			{
-				sA = sA + __shfl_xor_sync(0xFFFFFFFFu, sA, o);
-				sE = sE + __shfl_xor_sync(0xFFFFFFFFu, sE, o);
-				const float od = __shfl_xor_sync(0xFFFFFFFFu, dmax, o);
-				const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, imax, o);
-				if (oi != kInvalid && (imax == kInvalid || od > dmax || (od == dmax && oi < imax)))
-				{
-					dmax = od;
-					imax = oi;
-				}
+				const float od = __shfl_xor_sync(0xFFFFFFFFu, my.depth, o);
+				const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, my.hit, o);
+				deepest(my, od, oi, h0);
+				sum = sum + __shfl_xor_sync(0xFFFFFFFFu, sum, o);
 			}
-			const float D = h1 > h0 ? dmax : 0.0f;
 			if (lane == 0)
+			{
+				s_warp[warp] = my;
+				if (warp < 2)
+					s_sum[warp] = sum;
+			}
+			__syncthreads();
+			if (threadIdx.x == 0)
+			{
+				for (int w = 1; w < kWarps; w++)
+					deepest(my, s_warp[w].depth, s_warp[w].hit, h0);
+				s_block = my;
+			}
+			cluster.sync();
+			Deepest all = *cluster.map_shared_rank(&s_block, 0);
+			for (uint32_t b = 1; b < nb; b++)
+			{
+				const Deepest o = *cluster.map_shared_rank(&s_block, b);
+				deepest(all, o.depth, o.hit, h0);
+			}
+			const float sA = *cluster.map_shared_rank(s_sum, 0);
+			const float D = n ? all.depth : 0.0f;
+			if (rank == 0 && threadIdx.x == 0)
 			{
 				if (J_out)
 					J_out[c] = (sA * D) * D;
 				if (E_out)
-					E_out[c] = sE;
+					E_out[c] = s_sum[1];
 			}
-			if (!grad_dirs && !grad_x)
-				return;
-			const float gj = gJ ? gJ[c] : 0.0f, ge = gE ? gE[c] : 0.0f;
-			f3 gr = mk3(0.0f);
-			for (uint32_t i = h0 + lane; i < h1; i += 32)
+			double gr[3] = { 0.0, 0.0, 0.0 };
+			if (grad_dirs || grad_x)
 			{
-				const u26_prp_hit h = hits[i];
-				const HitGeo G = hit_geo(h, x, r);
-				float coef = 0.0f;
-				if (ge != 0.0f)
+				const float gj = gJ ? gJ[c] : 0.0f, ge = gE ? gE[c] : 0.0f;
+				// (64-bit: the index may pass 2^32 behind the last hit)
+				for (uint64_t i = uint64_t(h0) + rank * NT + threadIdx.x; i < h1; i += nb * NT)
 				{
-					const float kap = hit_kappa(h, vm);
-					if (kap > 1e-8f)
-						coef = ge * (2.0f * (G.delta + 3e-3f) / kap);
+					// without a cost gradient only the deepest hit has one
+					if (ge == 0.0f && uint32_t(i) != all.hit)
+						continue;
+					const u26_prp_hit h = hits[i];
+					const HitGeo G = hit_geo(h, x, r);
+					float coef = 0.0f;
+					if (ge != 0.0f)
+					{
+						const float kap = hit_kappa(h, vm);
+						if (kap > 1e-8f)
+							coef = ge * (2.0f * (G.delta + 3e-3f) / kap);
+					}
+					if (uint32_t(i) == all.hit && gj != 0.0f)
+						coef = coef + gj * (2.0f * sA * D);
+					if (coef == 0.0f)
+						continue;
+					const f3 g = G.n * (-G.delta * coef / G.rn);
+					gr[0] += double(g.x);
+					gr[1] += double(g.y);
+					gr[2] += double(g.z);
+					if (grad_x)
+					{
+						f3 gv[4];
+						delta_vertex_grads(h.type, G, r, coef, gv);
+#pragma unroll
+						for (int k = 0; k < 4; k++)
+							add3(grad_x, G.V[k], gv[k]);
+					}
 				}
-				if (i == imax && gj != 0.0f)
-					coef = coef + gj * (2.0f * sA * D);
-				if (coef == 0.0f)
-					continue;
-				gr = gr + G.n * (-G.delta * coef / G.rn);
-				if (grad_x)
+			}
+			if (grad_dirs)
+			{
+#pragma unroll
+				for (int k = 0; k < 3; k++)
 				{
-					f3 gv[4];
-					delta_vertex_grads(h.type, G, r, coef, gv);
 #pragma unroll
-					for (int k = 0; k < 4; k++)
-						add3(grad_x, G.V[k], gv[k]);
+					for (int o = 16; o >= 1; o >>= 1)
+						gr[k] += __shfl_xor_sync(0xFFFFFFFFu, gr[k], o);
+					if (lane == 0)
+						s_gr[warp][k] = gr[k];
+				}
+				__syncthreads();
+				if (threadIdx.x < 3)
+				{
+					double t = 0.0;
+					for (int w = 0; w < kWarps; w++)
+						t += s_gr[w][threadIdx.x];
+					s_gr_block[threadIdx.x] = t;
+				}
+				cluster.sync();
+				if (rank == 0 && threadIdx.x < 3)
+				{
+					double t = 0.0;
+					for (uint32_t b = 0; b < nb; b++)
+						t += cluster.map_shared_rank(s_gr_block, b)[threadIdx.x];
+					grad_dirs[3 * c + threadIdx.x] = float(t);
 				}
 			}
-#pragma unroll
-			for (int o = 16; o >= 1; o >>= 1)
-			{
-				gr.x = gr.x + __shfl_xor_sync(0xFFFFFFFFu, gr.x, o);
-				gr.y = gr.y + __shfl_xor_sync(0xFFFFFFFFu, gr.y, o);
-				gr.z = gr.z + __shfl_xor_sync(0xFFFFFFFFu, gr.z, o);
-			}
-			if (lane == 0 && grad_dirs)
-			{
-				grad_dirs[3 * c] = gr.x;
-				grad_dirs[3 * c + 1] = gr.y;
-				grad_dirs[3 * c + 2] = gr.z;
-			}
+			cluster.sync(); // no block leaves while another reads its shared memory
+		}
+
+		template <int NT>
+		cudaError_t launch_adjoint(cudaStream_t st, uint32_t nc, uint32_t blocks, const float* x, const u26_prp_hit* hits, const uint32_t* off,
+			const float* dirs, const float* va, const float* ea, const float* fa, const float* vm, float* J, float* E, const float* gJ,
+			const float* gE, float* grad_dirs, float* grad_x)
+		{
+			cudaLaunchConfig_t cfg = {};
+			cfg.gridDim = dim3(nc * blocks);
+			cfg.blockDim = dim3(NT);
+			cfg.stream = st;
+			cudaLaunchAttribute at[1];
+			at[0].id = cudaLaunchAttributeClusterDimension;
+			at[0].val.clusterDim.x = blocks;
+			at[0].val.clusterDim.y = 1;
+			at[0].val.clusterDim.z = 1;
+			cfg.attrs = at;
+			cfg.numAttrs = 1;
+			return cudaLaunchKernelEx(&cfg, adjoint_kernel<NT>, x, hits, off, dirs, va, ea, fa, vm, J, E, gJ, gE, grad_dirs, grad_x);
 		}
 	} // namespace
 } // namespace u26
@@ -237,7 +366,16 @@ U26_API u26_status u26_prp_adjoint(u26_ctx* ctx, const float* x, const u26_prp_h
 		return U26_OK;
 	if (!x || !hits || !hit_offsets || !dirs || !vert_area || !edge_area || !face_area || !vert_mass)
 		return set_error(ctx, U26_ERR_INVALID_INPUT, "u26_prp_adjoint: null input");
-	adjoint_kernel<<<div_up(32 * num_contours, 256), 256, 0, ctx->stream>>>(x, hits, hit_offsets, num_contours, dirs, vert_area, edge_area,
-		face_area, vert_mass, J, E, grad_J, grad_E, grad_dirs, grad_x);
+	// Threads per contour by the number of contours (the hits per contour are known on the device
+	// only): up to 18 contours leave room for 8 SMs each; up to 148 for eight 256-thread blocks each
+	// (the chip holds 1,184 of them at 64 registers); beyond that a block per contour fills it.
+	cudaError_t e;
+	if (num_contours <= 18u)
+		e = launch_adjoint<1024>(ctx->stream, num_contours, 8, x, hits, hit_offsets, dirs, vert_area, edge_area, face_area, vert_mass, J, E, grad_J,
+			grad_E, grad_dirs, grad_x);
+	else
+		e = launch_adjoint<256>(ctx->stream, num_contours, num_contours <= 148u ? 8u : 1u, x, hits, hit_offsets, dirs, vert_area, edge_area,
+			face_area, vert_mass, J, E, grad_J, grad_E, grad_dirs, grad_x);
+	U26_CUDA(ctx, e);
 	return after_launch(ctx, "adjoint_kernel");
 }
