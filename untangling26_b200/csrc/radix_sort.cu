@@ -13,9 +13,9 @@
 //    eight tiles at a time), and the keys go out in digit order from shared memory.
 //  Each pass reads and writes every pair once. The three-launch form (below) reads the keys twice, writes
 //  them uncoalesced and scans a count table in between; a sort of a few thousand keys is
-//  nothing but its launches (12 to 20 for 4 passes, now 1 or 6). Device time: 3,844 keys in 4 passes
-//  58 us, 25 us; 2.6 M and 3.9 M keys in 4 passes each 0.90 ms, 0.42 ms (a pass's 24 bytes a pair would
-//  take 12 us of the 46: the first wave's look-back and the ranking's shuffles are the rest).
+//  nothing but its launches (12 to 20 for 4 passes, now 1 or 6). Device time: 782 keys in 4 passes
+//  61 us, 10 us; 3,844 keys 58 us, 24 us; 2.6 M and 3.9 M keys in 4 passes each 0.90 ms, 0.42 ms (a pass's 24
+//  bytes a pair would take 12 us of the 46; the rest is a tile's chain of ranking rounds).
 // RadixSorter::sort_into (allocation-free callers: fixed scratch) and sorts of 2^30 keys and more (beyond
 // the look-back words' 30-bit counts) run three launches per digit: (1) per-tile digit
 // histogram, (2) exclusive scan of the digit-major count table (reduce / scan block sums /
@@ -270,13 +270,15 @@ namespace u26
 			}
 		}
 
-		// ---- one block: all digit passes of up to kSmall keys in shared memory
-		constexpr uint32_t kSmallThreads = 1024, kSmallItems = 8, kSmall = kSmallThreads * kSmallItems;
+		// ---- one block: all digit passes of up to kSmall keys in shared memory. NT threads: 256 up to 2,048 keys (the
+		// digit table has a row per warp to clear and scan), else 1,024; every thread holds ceil(n / NT) keys.
+		constexpr uint32_t kSmallItems = 8, kSmall = 1024 * kSmallItems, kSmallFew = 256 * kSmallItems;
+		template <uint32_t NT>
 		struct SmallSort
 		{
-			uint64_t keys[kSmall];
-			uint32_t vals[kSmall];
-			uint16_t cnt[32][256]; // per warp and digit
+			uint64_t keys[NT * kSmallItems];
+			uint32_t vals[NT * kSmallItems];
+			uint16_t cnt[NT / 32][256]; // per warp and digit
 			uint32_t start[256];
 			uint32_t warp_sum[8];
 		};
@@ -301,24 +303,27 @@ namespace u26
 				base += w < warp ? warp_sum[w] : 0u;
 			return base + s - v;
 		}
-		__global__ void __launch_bounds__(kSmallThreads) radix_small_kernel(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n,
+		template <uint32_t NT>
+		__global__ void __launch_bounds__(NT) radix_small_kernel(uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n,
 			int bit_lo, int bit_hi)
 		{
 			extern __shared__ __align__(16) unsigned char s_raw[];
-			SmallSort& S = *reinterpret_cast<SmallSort*>(s_raw);
+			SmallSort<NT>& S = *reinterpret_cast<SmallSort<NT>*>(s_raw);
 			const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
 			const uint32_t lt = (1u << lane) - 1u;
-			// a warp's keys are consecutive: item i of lane l is key 256 * warp + 32 * i + l
-			const uint32_t first = warp * 32u * kSmallItems + lane;
+			// a warp's keys are consecutive: item i of lane l is key 32 * (per * warp + i) + l
+			const uint32_t per = (n + NT - 1u) / NT;
+			const uint32_t first = warp * 32u * per + lane;
 			uint64_t k[kSmallItems];
 			uint32_t v[kSmallItems];
 #pragma unroll
 			for (uint32_t i = 0; i < kSmallItems; i++)
-			{
-				const uint32_t at = first + 32u * i;
-				k[i] = at < n ? keys[at] : 0u;
-				v[i] = at < n ? vals[at] : 0u;
-			}
+				if (i < per)
+				{
+					const uint32_t at = first + 32u * i;
+					k[i] = at < n ? keys[at] : 0u;
+					v[i] = at < n ? vals[at] : 0u;
+				}
 			for (int shift = bit_lo; shift < bit_hi; shift += 8)
 			{
 				const uint32_t mask = (1u << min(8, bit_hi - shift)) - 1u;
@@ -329,6 +334,8 @@ namespace u26
 #pragma unroll
 				for (uint32_t i = 0; i < kSmallItems; i++)
 				{
+					if (i >= per)
+						break;
 					const bool ok = first + 32u * i < n;
 					const uint32_t d = ok ? uint32_t(k[i] >> shift) & mask : 0x100u + lane;
 					const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
@@ -345,12 +352,15 @@ namespace u26
 				uint32_t total = 0;
 				if (tid < 256u)
 				{
-#pragma unroll 8
-					for (uint32_t w = 0; w < 32u; w++)
+					uint32_t c[NT / 32];
+#pragma unroll
+					for (uint32_t w = 0; w < NT / 32; w++)
+						c[w] = S.cnt[w][tid];
+#pragma unroll
+					for (uint32_t w = 0; w < NT / 32; w++)
 					{
-						const uint32_t t = S.cnt[w][tid];
 						S.cnt[w][tid] = uint16_t(total);
-						total += t;
+						total += c[w];
 					}
 				}
 				const uint32_t start = scan256(total, S.warp_sum);
@@ -359,7 +369,7 @@ namespace u26
 				__syncthreads();
 #pragma unroll
 				for (uint32_t i = 0; i < kSmallItems; i++)
-					if (first + 32u * i < n)
+					if (i < per && first + 32u * i < n)
 					{
 						const uint32_t d = uint32_t(k[i] >> shift) & mask;
 						const uint32_t at = S.start[d] + S.cnt[warp][d] + rank[i];
@@ -371,7 +381,7 @@ namespace u26
 				for (uint32_t i = 0; i < kSmallItems; i++)
 				{
 					const uint32_t at = first + 32u * i;
-					if (at < n)
+					if (i < per && at < n)
 					{
 						k[i] = S.keys[at];
 						v[i] = S.vals[at];
@@ -382,7 +392,7 @@ namespace u26
 			for (uint32_t i = 0; i < kSmallItems; i++)
 			{
 				const uint32_t at = first + 32u * i;
-				if (at < n)
+				if (i < per && at < n)
 				{
 					keys[at] = k[i];
 					vals[at] = v[i];
@@ -396,6 +406,7 @@ namespace u26
 		constexpr uint32_t kSweepHead = kMaxPasses * 256u + 64u;
 		constexpr uint32_t kAggregate = 0x40000000u, kInclusive = 0x80000000u, kCountMask = 0x3FFFFFFFu;
 		constexpr uint32_t kMaxPolls = 1u << 24;
+		constexpr int kLookBack = 8; // tiles looked up at a time (32: the same time)
 
 		// every pass's digit counts, and the look-back words cleared
 		__global__ void __launch_bounds__(256) radix_count_kernel(const uint64_t* __restrict__ keys, uint32_t n, int bit_lo, int bit_hi,
@@ -518,12 +529,13 @@ namespace u26
 			bool done = tile == 0;
 			while (!done)
 			{
-				uint32_t w[8];
+				// (the first wave's tiles find no total but tile 0's and walk back to it)
+				uint32_t w[kLookBack];
 #pragma unroll
-				for (int j = 0; j < 8; j++)
+				for (int j = 0; j < kLookBack; j++)
 					w[j] = t - j >= 0 ? *(volatile uint32_t*)(status + size_t(t - j) * 256u + tid) : uint32_t(kInclusive);
 #pragma unroll
-				for (int j = 0; j < 8; j++)
+				for (int j = 0; j < kLookBack; j++)
 				{
 					if (done || w[j] == 0u)
 						break;
@@ -638,15 +650,20 @@ namespace u26
 			return U26_OK;
 		if (n <= kSmall)
 		{
-			// one block: 3,844 keys in 4 passes take 25 us of device time, the tiled form's launches 50 to 60
-			static std::atomic<bool> sized[64];
-			if (ctx->device < 0 || ctx->device >= 64 || !sized[ctx->device].load(std::memory_order_acquire))
+			// one block
+			if (n <= kSmallFew)
+				radix_small_kernel<256><<<1, 256, sizeof(SmallSort<256>), ctx->stream>>>(keys, vals, n, bit_lo, bit_hi);
+			else
 			{
-				U26_CUDA(ctx, cudaFuncSetAttribute(radix_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SmallSort))));
-				if (ctx->device >= 0 && ctx->device < 64)
-					sized[ctx->device].store(true, std::memory_order_release);
+				static std::atomic<bool> sized[64];
+				if (ctx->device < 0 || ctx->device >= 64 || !sized[ctx->device].load(std::memory_order_acquire))
+				{
+					U26_CUDA(ctx, cudaFuncSetAttribute(radix_small_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SmallSort<1024>))));
+					if (ctx->device >= 0 && ctx->device < 64)
+						sized[ctx->device].store(true, std::memory_order_release);
+				}
+				radix_small_kernel<1024><<<1, 1024, sizeof(SmallSort<1024>), ctx->stream>>>(keys, vals, n, bit_lo, bit_hi);
 			}
-			radix_small_kernel<<<1, kSmallThreads, sizeof(SmallSort), ctx->stream>>>(keys, vals, n, bit_lo, bit_hi);
 			return after_launch(ctx, "radix_small_kernel");
 		}
 		U26_CUDA(ctx, keys_alt.reserve(sizeof(uint64_t) * n));
