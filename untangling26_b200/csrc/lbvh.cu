@@ -10,8 +10,6 @@
 // that the stack-overflow cut-off drops the same pairs.
 #include <algorithm>
 
-#include <cuda/atomic>
-
 #include "lbvh_internal.h"
 
 namespace u26
@@ -61,52 +59,13 @@ namespace u26
 			return v;
 		}
 
-		// Per-256 block AABB of the primitives (fn_reduce_*_tree_global_aabb). Lanes past n
-		// contribute +-inf, which leaves the block AABB of the valid leaves unchanged.
-		template <int TYPE>
-		__global__ void __launch_bounds__(256) reduce_blocks_kernel(const float* __restrict__ x, const uint32_t* __restrict__ prims,
-			uint32_t n, float* __restrict__ block_aabb)
+		// Global AABB of the first n primitives (fn_reduce_*_tree_global_aabb and fn_reduce_aabb_2_pass: minima and
+		// maxima, so any grouping gives the same values). One launch: every block reduces its
+		// stride, the last block to finish the blocks' results. arrivals is zero on entry
+		// and left zero.
+		constexpr uint32_t kReduceBlocks = 148u * 4u;
+		__device__ __forceinline__ void block_aabb_reduce(float (&v)[6], float (*s)[8])
 		{
-			__shared__ float s[6][8];
-			const uint32_t lid = blockIdx.x * 256u + threadIdx.x;
-			f3 mn = mk3(INFINITY), mx = mk3(-INFINITY);
-			if (lid < n)
-			{
-				f3 c;
-				prim_center_aabb<TYPE>(x, prims, lid, c, mn, mx);
-			}
-			float v[6] = { warp_min(mn.x), warp_min(mn.y), warp_min(mn.z), warp_max(mx.x), warp_max(mx.y), warp_max(mx.z) };
-			const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-			if (lane == 0)
-				for (int k = 0; k < 6; k++)
-					s[k][warp] = v[k];
-			__syncthreads();
-			if (warp == 0)
-			{
-				float r[6];
-				for (int k = 0; k < 6; k++)
-				{
-					float t = lane < 8 ? s[k][lane] : (k < 3 ? INFINITY : -INFINITY);
-					r[k] = k < 3 ? warp_min(t) : warp_max(t);
-				}
-				if (lane == 0)
-					for (int k = 0; k < 6; k++)
-						block_aabb[6 * blockIdx.x + k] = r[k];
-			}
-		}
-
-		// Second pass (fn_reduce_aabb_2_pass[_atomic]) over the first `nb` block AABBs.
-		__global__ void __launch_bounds__(256) reduce_final_kernel(const float* __restrict__ block_aabb, uint32_t nb, float* __restrict__ out)
-		{
-			__shared__ float s[6][8];
-			float v[6] = { INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY };
-			for (uint32_t b = threadIdx.x; b < nb; b += 256)
-			{
-				for (int k = 0; k < 3; k++)
-					v[k] = fminf(v[k], block_aabb[6 * b + k]);
-				for (int k = 3; k < 6; k++)
-					v[k] = fmaxf(v[k], block_aabb[6 * b + k]);
-			}
 			for (int k = 0; k < 6; k++)
 				v[k] = k < 3 ? warp_min(v[k]) : warp_max(v[k]);
 			const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -115,14 +74,50 @@ namespace u26
 					s[k][warp] = v[k];
 			__syncthreads();
 			if (warp == 0)
-			{
 				for (int k = 0; k < 6; k++)
 				{
-					float t = lane < 8 ? s[k][lane] : (k < 3 ? INFINITY : -INFINITY);
-					t = k < 3 ? warp_min(t) : warp_max(t);
-					if (lane == 0)
-						out[k] = t;
+					const float t = lane < 8 ? s[k][lane] : (k < 3 ? INFINITY : -INFINITY);
+					v[k] = k < 3 ? warp_min(t) : warp_max(t);
 				}
+		}
+		template <int TYPE>
+		__global__ void __launch_bounds__(256) reduce_aabb_kernel(const float* __restrict__ x, const uint32_t* __restrict__ prims,
+			uint32_t n, float* __restrict__ block_aabb, uint32_t* __restrict__ arrivals, float* __restrict__ out)
+		{
+			__shared__ float s[6][8];
+			__shared__ bool s_last;
+			float v[6] = { INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY };
+			for (uint64_t lid = uint64_t(blockIdx.x) * 256u + threadIdx.x; lid < n; lid += uint64_t(gridDim.x) * 256u)
+			{
+				f3 c, mn, mx;
+				prim_center_aabb<TYPE>(x, prims, uint32_t(lid), c, mn, mx);
+				const float p[6] = { mn.x, mn.y, mn.z, mx.x, mx.y, mx.z };
+				for (int k = 0; k < 6; k++)
+					v[k] = k < 3 ? fminf(v[k], p[k]) : fmaxf(v[k], p[k]);
+			}
+			block_aabb_reduce(v, s);
+			if (threadIdx.x == 0)
+			{
+				for (int k = 0; k < 6; k++)
+					block_aabb[6 * blockIdx.x + k] = v[k];
+				__threadfence();
+				s_last = atomicAdd(arrivals, 1u) == gridDim.x - 1u;
+			}
+			__syncthreads();
+			if (!s_last)
+				return;
+			__threadfence();
+			for (int k = 0; k < 6; k++)
+				v[k] = k < 3 ? INFINITY : -INFINITY;
+			for (uint32_t b = threadIdx.x; b < gridDim.x; b += 256u)
+				for (int k = 0; k < 6; k++)
+					v[k] = k < 3 ? fminf(v[k], __ldcg(block_aabb + 6 * b + k)) : fmaxf(v[k], __ldcg(block_aabb + 6 * b + k));
+			block_aabb_reduce(v, s);
+			if (threadIdx.x == 0)
+			{
+				for (int k = 0; k < 6; k++)
+					out[k] = v[k];
+				*arrivals = 0u;
 			}
 		}
 
@@ -147,9 +142,11 @@ namespace u26
 		// fn_compute_mortons: key = morton32(normalised centre) << 32 | leaf id; value = leaf id.
 		template <int TYPE>
 		__global__ void __launch_bounds__(256) morton_kernel(const float* __restrict__ x, const uint32_t* __restrict__ prims, uint32_t n,
-			const float* __restrict__ gaabb, uint64_t* __restrict__ keys, uint32_t* __restrict__ vals)
+			const float* __restrict__ gaabb, uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* __restrict__ health)
 		{
 			const uint32_t lid = blockIdx.x * blockDim.x + threadIdx.x;
+			if (lid == 0)
+				*health = 1u;
 			if (lid >= n)
 				return;
 			const f3 mn = mk3(gaabb[0], gaabb[1], gaabb[2]);
@@ -163,28 +160,6 @@ namespace u26
 			vals[lid] = lid;
 		}
 
-		// fn_reset_tree + fn_apply_sorted.
-		__global__ void __launch_bounds__(256) apply_sorted_kernel(const uint32_t* __restrict__ sorted_vals, uint32_t n,
-			uint2* __restrict__ children, uint32_t* __restrict__ object_idx, uint32_t* __restrict__ parent,
-			uint32_t* __restrict__ health)
-		{
-			const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-			const uint32_t ni = n - 1;
-			if (i == 0)
-			{
-				parent[0] = kInvalid;
-				*health = 1u;
-			}
-			if (i < ni)
-				object_idx[i] = kInvalid;
-			if (i < n)
-			{
-				const uint32_t orig = sorted_vals[i];
-				children[ni + i] = make_uint2(orig, orig);
-				object_idx[ni + i] = orig;
-			}
-		}
-
 		__device__ __forceinline__ int cp_ij(const uint64_t* __restrict__ keys, uint64_t mi, int j, int n)
 		{
 			if (j < 0 || j >= n)
@@ -192,14 +167,54 @@ namespace u26
 			return __clzll(mi ^ __ldg(keys + j));
 		}
 
-		// fn_build_inner_nodes: determineRange + findSplit (Karras 2012) over unique keys.
-		__global__ void __launch_bounds__(256) karras_kernel(const uint64_t* __restrict__ keys, uint32_t n, uint2* __restrict__ children,
-			uint32_t* __restrict__ parent, uint32_t* __restrict__ node_range)
+		constexpr uint32_t kTreelet = 1024;
+		constexpr uint32_t kTopRoot = 0x80000000u;
+		constexpr uint32_t kMaxHeight = 64;
+		// Device state of the refit plan while construct_tree makes it (one memset clears head and
+		// root_bits). Entry capacities: cap, see plan_capacity.
+		struct Plan
+		{
+			uint32_t* head;		  // [0] top nodes, [1] treelets, [2] chunks
+			uint32_t* root_bits;  // a bit per leaf: a treelet starts here
+			uint2* root_at;		  // by first leaf: the treelet's root node (then its index) and its parent's place in top_list
+			uint32_t* top_at;	  // by node: a top node's place in top_list
+			uint32_t* top_list;	  // top nodes, in no order
+			uint2* top_raw;		  // their children: a node, or kTopRoot | a treelet's first leaf
+			uint32_t* lo;		  // [cap + 1] the treelets' first leaves, then n
+			uint32_t* jump[2];	  // [cap + 1]
+			uint32_t* flag;		  // [cap + 1]
+			uint32_t cap;
+		};
+
+		// fn_reset_tree, fn_apply_sorted and fn_build_inner_nodes: determineRange + findSplit (Karras
+		// 2012) over unique keys. A thread per leaf: the leaf's links and primitive (the table in
+		// leaf order, for the refits' coalesced reads), and inner node i. A node of more than kTreelet
+		// leaves joins the top nodes and marks its children of at most kTreelet leaves as treelets.
+		template <int K>
+		__global__ void __launch_bounds__(256) karras_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ sorted_vals, uint32_t n,
+			const uint32_t* __restrict__ prims, uint32_t* __restrict__ leaf_prims, uint2* __restrict__ children, uint32_t* __restrict__ object_idx,
+			uint32_t* __restrict__ parent, uint32_t* __restrict__ node_range, Plan plan)
 		{
 			const int nid = blockIdx.x * blockDim.x + threadIdx.x;
 			const int num_inner = int(n) - 1;
+			if (nid >= int(n))
+				return;
+			{
+				const uint32_t orig = sorted_vals[nid];
+				children[num_inner + nid] = make_uint2(orig, orig);
+				object_idx[num_inner + nid] = orig;
+				if (K > 0)
+				{
+#pragma unroll
+					for (int k = 0; k < K; k++)
+						leaf_prims[size_t(K) * nid + k] = prims[size_t(K) * orig + k];
+				}
+			}
+			if (nid == 0)
+				parent[0] = kInvalid;
 			if (nid >= num_inner)
 				return;
+			object_idx[nid] = kInvalid;
 			int i = 0, j = num_inner;
 			if (nid != 0)
 			{
@@ -243,8 +258,34 @@ namespace u26
 						break;
 				}
 			}
-			int c_left = (min(i, j) == split) ? num_inner + split : split;
-			int c_right = (max(i, j) == split + 1) ? num_inner + split + 1 : split + 1;
+			int c_left = (lo == split) ? num_inner + split : split;
+			int c_right = (hi == split + 1) ? num_inner + split + 1 : split + 1;
+			if (hi - lo + 1 > int(kTreelet))
+			{
+				const uint32_t k = atomicAdd(plan.head, 1u);
+				auto child = [&](int first, int last, int c)
+				{
+					if (last - first + 1 > int(kTreelet))
+						return uint32_t(c);
+					atomicOr(plan.root_bits + (first >> 5), 1u << (first & 31));
+					plan.root_at[first] = make_uint2(uint32_t(c), k);
+					return kTopRoot | uint32_t(first);
+				};
+				uint2 raw = make_uint2(child(lo, split, c_left), child(split + 1, hi, c_right));
+				if (c_right >= num_inner)
+					raw = make_uint2(raw.y, raw.x); // as the links below
+				plan.top_at[nid] = k;
+				if (k < plan.cap)
+				{
+					plan.top_list[k] = uint32_t(nid);
+					plan.top_raw[k] = raw;
+				}
+			}
+			else if (nid == 0)
+			{
+				plan.root_bits[0] = 1u;
+				plan.root_at[0] = make_uint2(0u, kInvalid);
+			}
 			if (c_right >= num_inner)
 			{
 				const int tmp = c_left;
@@ -257,16 +298,15 @@ namespace u26
 			node_range[nid] = uint32_t(j);
 		}
 
-		// fn_check_construction.
-		__global__ void __launch_bounds__(256) check_kernel(const uint2* __restrict__ children, const uint32_t* __restrict__ parent, uint32_t ni,
-			uint32_t* __restrict__ health)
+		// ld3 as an 8-byte and a 4-byte load (which two words share 8 bytes depends on the vertex): a gather's L1
+		// wavefronts are its lanes' lines times its loads.
+		__device__ __forceinline__ f3 ld3_pair(const float* __restrict__ p, uint32_t i)
 		{
-			const uint32_t nid = blockIdx.x * blockDim.x + threadIdx.x;
-			if (nid >= ni)
-				return;
-			const uint2 c = children[nid];
-			if (parent[c.x] != nid || parent[c.y] != nid)
-				*health = 0u;
+			const float* v = p + 3 * i;
+			const bool low = (reinterpret_cast<uintptr_t>(v) & 4u) == 0u; // (x, y), z; else x, (y, z)
+			const float2 two = __ldg(reinterpret_cast<const float2*>(low ? v : v + 1));
+			const float one = __ldg(low ? v + 2 : v);
+			return low ? mk3(two.x, two.y, one) : mk3(one, two.x, two.y);
 		}
 
 		template <int TYPE>
@@ -280,7 +320,7 @@ namespace u26
 			if constexpr (TYPE == U26_TREE_FACE)
 			{
 				const uint32_t a = __ldg(prims + 3 * pid), b = __ldg(prims + 3 * pid + 1), c = __ldg(prims + 3 * pid + 2);
-				const f3 s0 = ld3(x0, a), s1 = ld3(x0, b), s2 = ld3(x0, c);
+				const f3 s0 = ld3_pair(x0, a), s1 = ld3_pair(x0, b), s2 = ld3_pair(x0, c);
 				if (same)
 				{
 					mn = vmin(s0, vmin(s1, s2));
@@ -288,7 +328,7 @@ namespace u26
 				}
 				else
 				{
-					const f3 e0 = ld3(x1, a), e1 = ld3(x1, b), e2 = ld3(x1, c);
+					const f3 e0 = ld3_pair(x1, a), e1 = ld3_pair(x1, b), e2 = ld3_pair(x1, c);
 					mn = vmin(vmin(s0, vmin(s1, s2)), vmin(e0, vmin(e1, e2)));
 					mx = vmax(vmax(s0, vmax(s1, s2)), vmax(e0, vmax(e1, e2)));
 				}
@@ -297,7 +337,7 @@ namespace u26
 			else if constexpr (TYPE == U26_TREE_EDGE)
 			{
 				const uint32_t a = __ldg(prims + 2 * pid), b = __ldg(prims + 2 * pid + 1);
-				const f3 s0 = ld3(x0, a), s1 = ld3(x0, b);
+				const f3 s0 = ld3_pair(x0, a), s1 = ld3_pair(x0, b);
 				if (same)
 				{
 					mn = vmin(s0, s1);
@@ -305,7 +345,7 @@ namespace u26
 				}
 				else
 				{
-					const f3 e0 = ld3(x1, a), e1 = ld3(x1, b);
+					const f3 e0 = ld3_pair(x1, a), e1 = ld3_pair(x1, b);
 					mn = vmin(vmin(s0, s1), vmin(e0, e1));
 					mx = vmax(vmax(s0, s1), vmax(e0, e1));
 				}
@@ -313,7 +353,7 @@ namespace u26
 			}
 			else
 			{
-				const f3 s0 = ld3(x0, pid);
+				const f3 s0 = ld3_pair(x0, pid);
 				if (same)
 				{
 					mn = s0;
@@ -321,7 +361,7 @@ namespace u26
 				}
 				else
 				{
-					const f3 e0 = ld3(x1, pid);
+					const f3 e0 = ld3_pair(x1, pid);
 					mn = vmin(s0, e0);
 					mx = vmax(s0, e0);
 				}
@@ -350,185 +390,355 @@ namespace u26
 		}
 
 		// Bottom-up union (fn_refit_tree_aabb, lbvh.cpp:694-758) without atomics or waits, level
-		// by level. construct_tree prepares, once per topology:
-		//  * the height of every inner node (1 + the larger child height, leaves 0); a Karras
-		//    tree over unique 64-bit keys is at most 64 deep, so a height fits a byte;
+		// by level. construct_tree prepares, once per topology and without a host round trip:
 		//  * treelets: the maximal subtrees of at most kTreelet leaves (each a contiguous leaf
 		//    range, Karras 2012), packed in leaf order into chunks of at most kTreelet leaves;
+		//  * for every inner node of a chunk one word: both children as chunk-local slots and
+		//    its height (1 + the larger child height, leaves 0; a Karras tree over unique
+		//    64-bit keys is at most 64 deep);
 		//  * the top nodes (more than kTreelet leaves) sorted by height, their children as
 		//    compact ids (top node j, or 0x80000000 | treelet b).
-		// refit_chunk_kernel: one block per chunk. Leaf boxes, the chunk's inner nodes (child
-		// links and heights) and their boxes live in shared memory; the nodes of height h are
+		// refit_chunk_kernel: one block per chunk. Leaf boxes, the chunk's inner nodes' words
+		// and their boxes live in shared memory; the nodes of height h are
 		// united in step h, after a barrier, so every union reads finished children without
 		// atomics or fences. Boxes go out coalesced.
-		// refit_top_kernel: one block for the top tree. The treelet roots' boxes are read once,
-		// then the top nodes height by height, in shared memory when the tree fits, else
-		// through L2.
+		// refit_top_kernel: one block for the top tree, height by height, in shared memory when
+		// it fits, else through L2.
 		// Unions keep the (first child, second child) operand order of the reference.
-		constexpr uint32_t kTreelet = 1024;
-		constexpr uint32_t kTopRoot = 0x80000000u;
-		constexpr uint32_t kMaxHeight = 64;
-		constexpr size_t kTopSharedBytes = 226u * 1024u; // the top tree in shared memory up to this size (227 KB per block, less static)
+		// The plan's counts stay on the device and its arrays have their upper bounds' sizes from
+		// the start, so a construction is 9 to 14 launches without an allocation or a host read (heights by
+		// device atomics over the whole tree, two sorts and two host reads made it 53 to 61). Face and edge
+		// tree constructed and refit: 3,844 triangles 1.80 ms, 0.18 ms now (host and launch latency); 130,050
+		// 1.85 ms, 0.29 ms; 2.6 M 3.5 ms, 1.45 ms (0.43 ms of it the sorts, 0.31 ms the one-block kernels).
 		constexpr size_t kChunkSmem = 2 * 24 * kTreelet + sizeof(uint32_t) * kTreelet;
-		struct Box6
-		{
-			float v[6];
-		};
-		__device__ __forceinline__ Box6 unite(const Box6& a, const Box6& b)
-		{
-			return Box6{ { fminf(a.v[0], b.v[0]), fminf(a.v[1], b.v[1]), fminf(a.v[2], b.v[2]), fmaxf(a.v[3], b.v[3]), fmaxf(a.v[4], b.v[4]),
-				fmaxf(a.v[5], b.v[5]) } };
-		}
-		__device__ __forceinline__ void store_box6(NodeBox* p, const Box6& b, float w_mx)
-		{
-			__stcg(&p->mn, make_float4(b.v[0], b.v[1], b.v[2], 0.0f));
-			__stcg(&p->mx, make_float4(b.v[3], b.v[4], b.v[5], w_mx));
-		}
-		__device__ __forceinline__ Box6 load_box6(const NodeBox* p)
-		{
-			const float4 a = __ldcg(&p->mn), b = __ldcg(&p->mx);
-			return Box6{ { a.x, a.y, a.z, b.x, b.y, b.z } };
-		}
-		// leaf order -> primitive table, permuted once per construction
-		template <int K>
-		__global__ void __launch_bounds__(256) permute_prims_kernel(const uint32_t* __restrict__ sorted_get_original,
-			const uint32_t* __restrict__ prims, uint32_t n, uint32_t* __restrict__ out)
-		{
-			const uint32_t lid = blockIdx.x * blockDim.x + threadIdx.x;
-			if (lid >= n)
-				return;
-			const uint32_t p = sorted_get_original[lid];
-#pragma unroll
-			for (int k = 0; k < K; k++)
-				out[size_t(K) * lid + k] = prims[size_t(K) * p + k];
-		}
 
-		// ---- construction: heights, treelets, top nodes
-		// heights: a thread per leaf climbs; at each inner node the first arrival stops and the
-		// second (acquiring the first's height) stores 1 + the larger child height. counters are
-		// zero on entry. Bounded by the tree depth (<= 64 levels, capped at kMaxClimb).
-		__global__ void __launch_bounds__(256) height_kernel(const uint32_t* __restrict__ parent, const uint2* __restrict__ children, uint32_t n,
-			uint32_t* __restrict__ counters, uint8_t* __restrict__ height, uint32_t* __restrict__ health)
+		// Top nodes lie above nodes of more than kTreelet leaves, disjoint at every depth, and a tree over
+		// 30 Morton bits and the leaf id bits has at most 62 depths with one: at most 62 n / 1025 < n / 16
+		// top nodes, and one more treelet.
+		inline uint32_t plan_capacity(uint32_t n) { return n / 16u + 64u; }
+		// Two consecutive chunks hold more than kTreelet leaves together.
+		inline uint32_t chunk_bound(uint32_t n) { return 2u * (n / kTreelet) + 2u; }
+
+		// ---- construction: treelets and chunks (one block)
+		__device__ __forceinline__ uint32_t block_scan1024(uint32_t v, uint32_t* warp_sum, uint32_t& total)
 		{
-			const uint32_t lid = blockIdx.x * blockDim.x + threadIdx.x;
-			if (lid >= n)
-				return;
-			const uint32_t ni = n - 1;
-			uint32_t node = parent[ni + lid];
-			uint32_t steps = 0;
-			while (node != kInvalid)
+			const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+			uint32_t s = v;
+#pragma unroll
+			for (int o = 1; o < 32; o <<= 1)
 			{
-				if (++steps > 100000u || node >= ni)
+				const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, s, o);
+				s += lane >= uint32_t(o) ? t : 0u;
+			}
+			if (lane == 31u)
+				warp_sum[warp] = s;
+			__syncthreads();
+			uint32_t w = warp_sum[lane];
+			total = __reduce_add_sync(0xFFFFFFFFu, w);
+			w = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? w : 0u);
+			__syncthreads();
+			return w + s - v;
+		}
+		// Treelets in leaf order, then packed greedily into chunks of at most kTreelet leaves. The greedy
+		// chain (a chunk ends where the next treelet does not fit) is followed by doubling: jump[b] is the
+		// first treelet after a chunk that begins at b, and after round r every chunk start within
+		// 2^(r + 1) chunks of the first is flagged. (One thread walking the treelets took 0.3 ms for 3,913
+		// of them.)
+		constexpr uint32_t kChainShared = 12u * 1024u; // treelets and their end (192 KB)
+		__global__ void __launch_bounds__(1024) plan_chunks_kernel(Plan plan, uint32_t n, uint32_t* __restrict__ roots, uint32_t* __restrict__ chunk_lo,
+			uint32_t* __restrict__ chunk_tb, uint32_t max_chunks, uint32_t* __restrict__ info, uint32_t* __restrict__ health)
+		{
+			extern __shared__ __align__(16) uint32_t s_chain[]; // [4][treelets + 1]
+			__shared__ uint32_t s_sum[32];
+			const uint32_t t = threadIdx.x;
+			const uint32_t words = (n + 31u) / 32u;
+			uint32_t nt = 0;
+			constexpr uint32_t kPer = 8; // 16-byte loads a thread
+			for (uint32_t w0 = 0; w0 < words; w0 += 4096u * kPer)
+			{
+				uint4 w[kPer];
+				uint32_t sum = 0;
+#pragma unroll
+				for (uint32_t k = 0; k < kPer; k++)
 				{
-					atomicExch(health, 0u);
-					return;
+					const uint32_t i = w0 + (t * kPer + k) * 4u;
+					w[k] = i < words ? *reinterpret_cast<const uint4*>(plan.root_bits + i) : make_uint4(0u, 0u, 0u, 0u); // zero past the last leaf
+					sum += __popc(w[k].x) + __popc(w[k].y) + __popc(w[k].z) + __popc(w[k].w);
 				}
-				if (cuda::atomic_ref<uint32_t, cuda::thread_scope_device>(counters[node]).fetch_add(1u, cuda::memory_order_acq_rel) == 0u)
-					return;
-				const uint2 c = children[node];
-				// the sibling's height, ordered after its store by the arrival's acquire
-				const uint32_t ha = c.x >= ni ? 0u : height[c.x];
-				const uint32_t hb = c.y >= ni ? 0u : height[c.y];
-				const uint32_t h = 1u + max(ha, hb);
-				if (h > kMaxHeight)
+				uint32_t total;
+				uint32_t at = nt + block_scan1024(sum, s_sum, total);
+				nt += total;
+				if (sum)
 				{
-					atomicExch(health, 0u);
-					return;
+#pragma unroll
+					for (uint32_t k = 0; k < kPer; k++)
+#pragma unroll
+						for (uint32_t q = 0; q < 4; q++)
+						{
+							const uint32_t i = w0 + (t * kPer + k) * 4u + q;
+							for (uint32_t m = q == 0 ? w[k].x : q == 1 ? w[k].y : q == 2 ? w[k].z : w[k].w; m; m &= m - 1u, at++)
+								if (at < plan.cap)
+									plan.lo[at] = 32u * i + uint32_t(__ffs(m) - 1);
+						}
 				}
-				height[node] = uint8_t(h);
-				node = parent[node];
 			}
-		}
-		__device__ __forceinline__ uint32_t node_size(uint32_t x, uint32_t ni, const uint32_t* __restrict__ range)
-		{
-			if (x >= ni)
-				return 1u;
-			const uint32_t r = range[x];
-			return (x > r ? x - r : r - x) + 1u;
-		}
-		// treelet roots (key: first leaf) and top nodes (key: height, node) appended to two lists
-		__global__ void __launch_bounds__(256) treelet_mark_kernel(const uint32_t* __restrict__ parent, const uint32_t* __restrict__ range,
-			const uint8_t* __restrict__ height, uint32_t n, uint32_t* __restrict__ counts, uint64_t* __restrict__ top_keys,
-			uint32_t* __restrict__ top_vals, uint64_t* __restrict__ root_keys, uint32_t* __restrict__ root_vals)
-		{
-			const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-			const uint32_t ni = n - 1;
-			if (x >= 2 * n - 1)
-				return;
-			const uint32_t sz = node_size(x, ni, range);
-			if (sz > kTreelet)
+			const uint32_t m = plan.head[0];
+			if (nt == 0u || nt > plan.cap || m > plan.cap)
 			{
-				const uint32_t j = atomicAdd(counts + 0, 1u);
-				top_keys[j] = (uint64_t(height[x]) << 32) | x;
-				top_vals[j] = x;
+				// more nodes than a tree over distinct keys has: the refits find no chunk
+				if (t == 0)
+				{
+					info[0] = info[1] = info[2] = 0u;
+					atomicExch(health, 0u);
+				}
 				return;
 			}
-			const uint32_t p = parent[x];
-			if (p == kInvalid || node_size(p, ni, range) > kTreelet)
+			if (t == 0)
+				plan.lo[nt] = n;
+			__syncthreads();
+			for (uint32_t b = t; b < nt; b += 1024u)
 			{
-				const uint32_t lo = x >= ni ? x - ni : min(x, range[x]);
-				const uint32_t b = atomicAdd(counts + 1, 1u);
-				root_keys[b] = lo;
-				root_vals[b] = x;
+				const uint32_t first = plan.lo[b];
+				roots[b] = plan.root_at[first].x;
+				plan.root_at[first].x = b;
+			}
+			// the chain's arrays in shared memory when they fit
+			const uint32_t len = nt + 1u;
+			const bool fits = len <= kChainShared;
+			uint32_t* lo_ = fits ? s_chain : plan.lo;
+			uint32_t* jump = fits ? s_chain + len : plan.jump[0];
+			uint32_t* next = fits ? s_chain + 2u * len : plan.jump[1];
+			uint32_t* flag = fits ? s_chain + 3u * len : plan.flag;
+			if (fits)
+				for (uint32_t b = t; b <= nt; b += 1024u)
+					lo_[b] = plan.lo[b];
+			__syncthreads();
+			for (uint32_t b = t; b <= nt; b += 1024u)
+			{
+				// the last treelet b' > b with lo[b'] <= lo[b] + kTreelet
+				uint32_t lo = b, hi = nt + 1u;
+				const uint32_t end = b < nt ? lo_[b] + kTreelet : 0u;
+				if (b < nt)
+					while (hi - lo > 1u)
+					{
+						const uint32_t mid = (lo + hi) >> 1;
+						if (lo_[mid] <= end)
+							lo = mid;
+						else
+							hi = mid;
+					}
+				jump[b] = b < nt ? max(lo, b + 1u) : nt;
+				flag[b] = b == 0u ? 1u : 0u;
+			}
+			__syncthreads();
+			for (uint32_t reach = 1; reach < nt; reach <<= 1)
+			{
+				for (uint32_t b = t; b < nt; b += 1024u)
+					if (flag[b])
+						flag[jump[b]] = 1u;
+				for (uint32_t b = t; b <= nt; b += 1024u)
+					next[b] = jump[jump[b]];
+				__syncthreads();
+				uint32_t* x = jump;
+				jump = next;
+				next = x;
+			}
+			uint32_t k0 = 0;
+			for (uint32_t b0 = 0; b0 < nt; b0 += 1024u)
+			{
+				const uint32_t b = b0 + t;
+				const bool head = b < nt && flag[b];
+				uint32_t total;
+				const uint32_t k = k0 + block_scan1024(head ? 1u : 0u, s_sum, total);
+				k0 += total;
+				if (head && k < max_chunks)
+				{
+					chunk_lo[k] = lo_[b];
+					chunk_tb[k] = b;
+				}
+			}
+			if (t == 0)
+			{
+				const uint32_t k = min(k0, max_chunks);
+				chunk_lo[k] = n;
+				chunk_tb[k] = nt;
+				info[0] = m;
+				info[1] = nt;
+				info[2] = k;
 			}
 		}
-		// compact ids of the sorted lists, then each top node's children as compact ids, the end
-		// of each height's run, and the treelets' leaf ranges
-		__global__ void __launch_bounds__(256) treelet_map_kernel(const uint32_t* __restrict__ top_nodes, uint32_t m,
-			const uint32_t* __restrict__ roots, uint32_t nt, uint32_t* __restrict__ cmap)
+		// The words of a chunk's inner nodes: child slots (10 bits and a leaf bit each) and the height, 0 for a
+		// node whose leaves are not all in the chunk. Heights: a thread per leaf climbs inside the chunk; the
+		// first arrival at a node stops, the second stores 1 + the larger child height. Checks the
+		// parent links (fn_check_construction).
+		constexpr uint32_t kChunkThreads = 512;
+		__global__ void __launch_bounds__(kChunkThreads) plan_words_kernel(const uint32_t* __restrict__ parent, const uint2* __restrict__ children,
+			const uint32_t* __restrict__ node_range, uint32_t n, const uint32_t* __restrict__ chunk_lo, const uint32_t* __restrict__ chunk_tb,
+			const uint32_t* __restrict__ info, const uint32_t* __restrict__ roots, uint32_t* __restrict__ words, uint8_t* __restrict__ root_height,
+			uint32_t* __restrict__ health)
 		{
-			const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-			if (i < m)
-				cmap[top_nodes[i]] = i;
-			else if (i < m + nt)
-				cmap[roots[i - m]] = kTopRoot | (i - m);
-		}
-		__global__ void __launch_bounds__(256) treelet_links_kernel(const uint32_t* __restrict__ top_nodes, uint32_t m,
-			const uint2* __restrict__ children, const uint32_t* __restrict__ cmap, const uint8_t* __restrict__ height,
-			uint2* __restrict__ top_links, uint32_t* __restrict__ height_end, const uint32_t* __restrict__ roots, uint32_t nt,
-			const uint32_t* __restrict__ range, uint32_t n, uint32_t* __restrict__ root_size, uint8_t* __restrict__ top_height)
-		{
-			const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-			if (i < m)
+			__shared__ uint32_t s_word[kTreelet], s_parent[kTreelet], s_leaf_parent[kTreelet], s_count[kTreelet];
+			__shared__ volatile uint8_t s_height[kTreelet];
+			if (blockIdx.x >= info[2])
+				return;
+			const uint32_t base = chunk_lo[blockIdx.x], cnt = chunk_lo[blockIdx.x + 1] - base;
+			const uint32_t ni = n - 1u, t = threadIdx.x;
+			if (cnt > kTreelet || base + cnt > n)
 			{
-				const uint32_t x = top_nodes[i];
+				if (t == 0)
+					atomicExch(health, 0u);
+				return;
+			}
+			for (uint32_t k = t; k < cnt; k += kChunkThreads)
+			{
+				const uint32_t x = base + k;
+				uint32_t word = 0, par = kInvalid;
+				if (x < ni)
+				{
+					const uint32_t r = __ldg(node_range + x);
+					if (min(x, r) >= base && max(x, r) < base + cnt)
+					{
+						// children of a node inside the chunk are inside it too (checked, not assumed)
+						const uint2 c = __ldg(children + x);
+						const uint32_t ia = c.x >= ni ? c.x - ni - base : c.x - base, ib = c.y >= ni ? c.y - ni - base : c.y - base;
+						if (ia < cnt && ib < cnt)
+						{
+							word = 0x80000000u | (ia | (c.x >= ni ? 0x400u : 0u)) | ((ib | (c.y >= ni ? 0x400u : 0u)) << 11);
+							par = __ldg(parent + x);
+						}
+						else
+							atomicExch(health, 0u);
+					}
+				}
+				s_word[k] = word;
+				s_parent[k] = par;
+				s_leaf_parent[k] = __ldg(parent + ni + x);
+				s_count[k] = 0u;
+				s_height[k] = 0;
+			}
+			__syncthreads();
+			for (uint32_t k = t; k < cnt; k += kChunkThreads)
+			{
+				const uint32_t w = s_word[k], a = w & 0x7FFu, b = (w >> 11) & 0x7FFu;
+				if (w && ((a & 0x400u ? s_leaf_parent[a & 0x3FFu] : s_parent[a]) != base + k || (b & 0x400u ? s_leaf_parent[b & 0x3FFu] : s_parent[b]) != base + k))
+					atomicExch(health, 0u);
+				uint32_t node = s_leaf_parent[k];
+				for (uint32_t steps = 0; steps < kMaxHeight; steps++)
+				{
+					const uint32_t i = node - base; // kInvalid and nodes outside wrap past cnt
+					if (node == kInvalid || i >= cnt || s_word[i] == 0u)
+						break;
+					__threadfence_block();
+					if (atomicAdd(&s_count[i], 1u) == 0u)
+						break;
+					__threadfence_block();
+					const uint32_t w = s_word[i], a = w & 0x7FFu, b = (w >> 11) & 0x7FFu;
+					const uint32_t ha = (a & 0x400u) ? 0u : s_height[a & 0x3FFu], hb = (b & 0x400u) ? 0u : s_height[b & 0x3FFu];
+					s_height[i] = uint8_t(1u + max(ha, hb));
+					node = s_parent[i];
+				}
+			}
+			__syncthreads();
+			for (uint32_t k = t; k < cnt; k += kChunkThreads)
+				if (base + k < ni)
+				{
+					const uint32_t w = s_word[k];
+					if (w && s_height[k] == 0)
+						atomicExch(health, 0u); // unreached
+					words[base + k] = w ? (w & 0x3FFFFFu) | (uint32_t(s_height[k]) << 22) : 0u;
+				}
+			const uint32_t tb0 = chunk_tb[blockIdx.x], tb1 = chunk_tb[blockIdx.x + 1];
+			for (uint32_t b = tb0 + t; b < tb1; b += kChunkThreads)
+			{
+				const uint32_t x = roots[b];
+				const uint32_t k = x >= ni ? x - ni - base : x - base;
+				root_height[b] = x < ni && k < cnt ? s_height[k] : uint8_t(0);
+				if (k >= cnt)
+					atomicExch(health, 0u);
+			}
+		}
+		// The top nodes sorted by height with their children's compact ids (one block): heights climb from the treelet
+		// roots as in plan_words_kernel, then a counting sort over the heights.
+		struct TopScratch // words per top node
+		{
+			uint32_t height, count, parent, place;
+		};
+		constexpr uint32_t kTopScratchShared = 12u * 1024u; // top nodes whose scratch fits in shared memory (192 KB)
+		__global__ void __launch_bounds__(1024) plan_top_kernel(Plan plan, const uint32_t* __restrict__ parent, const uint2* __restrict__ children,
+			const uint32_t* __restrict__ info, const uint8_t* __restrict__ root_height, TopScratch* __restrict__ scratch,
+			uint32_t* __restrict__ top_nodes, uint2* __restrict__ top_links, uint32_t* __restrict__ root_slot,
+			uint32_t* __restrict__ level_end, uint32_t* __restrict__ health)
+		{
+			extern __shared__ __align__(16) unsigned char s_raw[];
+			__shared__ uint32_t s_level[kMaxHeight + 2];
+			const uint32_t t = threadIdx.x;
+			const uint32_t m = info[0], nt = info[1];
+			TopScratch* S = m <= kTopScratchShared ? reinterpret_cast<TopScratch*>(s_raw) : scratch;
+#pragma unroll 4
+			for (uint32_t j = t; j < m; j += 1024u)
+			{
+				const uint32_t x = plan.top_list[j];
 				const uint2 c = children[x];
-				top_links[i] = make_uint2(cmap[c.x], cmap[c.y]);
-				const uint32_t h = height[x];
-				top_height[i] = uint8_t(h);
-				if (i + 1 == m || height[top_nodes[i + 1]] != h)
-					height_end[h] = i + 1;
+				const uint32_t p = parent[x];
+				S[j] = TopScratch{ 0u, 0u, p == kInvalid ? kInvalid : plan.top_at[p], 0u };
+				if (parent[c.x] != x || parent[c.y] != x)
+					atomicExch(health, 0u);
 			}
-			if (i < nt)
-				root_size[i] = node_size(roots[i], n - 1, range);
-		}
-		// treelets (in leaf order) packed greedily into chunks of at most kTreelet leaves; one
-		// thread (a few thousand treelets)
-		// (chunk_tb: each chunk's first treelet, then nt)
-		__global__ void treelet_chunks_kernel(const uint32_t* __restrict__ root_size, uint32_t nt, uint32_t* __restrict__ chunk_lo,
-			uint32_t* __restrict__ chunk_tb, uint32_t* __restrict__ nchunks)
-		{
-			if (threadIdx.x != 0 || blockIdx.x != 0)
-				return;
-			uint32_t k = 0, lo = 0, fill = 0, tb = 0;
-			for (uint32_t b = 0; b < nt; b++)
+			if (t < kMaxHeight + 2)
+				s_level[t] = 0u;
+			__syncthreads();
+#pragma unroll 4
+			for (uint32_t b = t; b < nt; b += 1024u)
 			{
-				const uint32_t sz = root_size[b];
-				if (fill > 0 && fill + sz > kTreelet)
+				uint32_t j = m ? plan.root_at[plan.lo[b]].y : kInvalid;
+				uint32_t h = root_height[b];
+				for (uint32_t steps = 0; j < m && steps <= kMaxHeight; steps++)
 				{
-					chunk_tb[k] = tb;
-					chunk_lo[k++] = lo;
-					lo += fill;
-					fill = 0;
-					tb = b;
+					h++;
+					atomicMax(&S[j].height, h);
+					__threadfence_block();
+					if (atomicAdd(&S[j].count, 1u) == 0u)
+						break;
+					__threadfence_block();
+					h = atomicMax(&S[j].height, 0u);
+					j = S[j].parent;
 				}
-				fill += sz;
 			}
-			chunk_tb[k] = tb;
-			chunk_lo[k++] = lo;
-			chunk_lo[k] = lo + fill;
-			chunk_tb[k] = nt;
-			*nchunks = k;
+			__syncthreads();
+			for (uint32_t j = t; j < m; j += 1024u)
+			{
+				const uint32_t h = S[j].height;
+				if (h == 0u || h > kMaxHeight)
+					atomicExch(health, 0u);
+				atomicAdd(&s_level[min(h, kMaxHeight) + 1u], 1u);
+			}
+			__syncthreads();
+			if (t == 0)
+				for (uint32_t h = 1; h < kMaxHeight + 2; h++)
+					s_level[h] += s_level[h - 1]; // s_level[h]: first place of height h
+			__syncthreads();
+			if (t <= kMaxHeight)
+				level_end[t] = s_level[t + 1];
+			__syncthreads();
+			for (uint32_t j = t; j < m; j += 1024u)
+				S[j].place = atomicAdd(&s_level[min(S[j].height, kMaxHeight)], 1u);
+			__syncthreads();
+#pragma unroll 4
+			for (uint32_t j = t; j < m; j += 1024u)
+			{
+				const uint32_t place = S[j].place;
+				auto compact = [&](uint32_t v, uint32_t side)
+				{
+					if (!(v & kTopRoot))
+						return S[min(plan.top_at[v], m - 1u)].place;
+					const uint32_t r = plan.root_at[v & ~kTopRoot].x;
+					root_slot[min(r, nt - 1u)] = 2u * place + side;
+					return kTopRoot | r;
+				};
+				const uint2 raw = plan.top_raw[j];
+				top_links[place] = make_uint2(compact(raw.x, 0u), compact(raw.y, 1u));
+				top_nodes[S[j].place] = plan.top_list[j];
+			}
 		}
 
 		// ---- refit
@@ -554,22 +764,24 @@ namespace u26
 		}
 		// One 512-thread block per chunk of at most 1024 leaves, two leaves and two inner-node
 		// slots per thread, so that four chunks share an SM and one chunk's loads overlap another's
-		// height steps.
-		constexpr uint32_t kChunkThreads = 512;
+		// height steps. Bound by L1: the position gathers' wavefronts (82 % of its peak; 2.6 M faces, two position
+		// arrays: 110 us, where the bytes alone would take 45).
 		template <int TYPE, bool FUSED>
 		__global__ void __launch_bounds__(kChunkThreads, 4) refit_chunk_kernel(const uint32_t* __restrict__ sorted_get_original,
 			NodeBox* __restrict__ boxes, const float* __restrict__ x0, const float* __restrict__ x1, const float* __restrict__ thickness,
-			const uint32_t* __restrict__ prims, bool prims_in_leaf_order, const uint2* __restrict__ children,
-			const uint32_t* __restrict__ node_range, const uint8_t* __restrict__ height, const uint32_t* __restrict__ chunk_lo, uint32_t n,
-			const uint32_t* __restrict__ chunk_tb, const uint32_t* __restrict__ roots, SBox* __restrict__ root_box, uint32_t* __restrict__ health)
+			const uint32_t* __restrict__ prims, bool prims_in_leaf_order, const uint32_t* __restrict__ words,
+			const uint32_t* __restrict__ info, const uint32_t* __restrict__ chunk_lo, uint32_t n,
+			const uint32_t* __restrict__ chunk_tb, const uint32_t* __restrict__ roots, const uint32_t* __restrict__ root_slot,
+			SBox* __restrict__ root_box, uint32_t* __restrict__ health)
 		{
 			// dynamic shared memory (kChunkSmem bytes, four blocks per SM): leaf boxes, inner boxes,
-			// child links as two 16-bit chunk-local slots (bit 15: leaf)
+			// the nodes' words
 			extern __shared__ __align__(16) unsigned char s_raw[];
 			SBox* s_leaf = reinterpret_cast<SBox*>(s_raw);
 			SBox* s_inner = s_leaf + kTreelet;
-			uint32_t* s_child = reinterpret_cast<uint32_t*>(s_inner + kTreelet);
 			__shared__ uint32_t s_hmax;
+			if (blockIdx.x >= info[2])
+				return;
 			const uint32_t base = chunk_lo[blockIdx.x];
 			const uint32_t cnt = chunk_lo[blockIdx.x + 1] - base;
 			const uint32_t ni = n - 1;
@@ -583,30 +795,14 @@ namespace u26
 			}
 			if (t == 0)
 				s_hmax = 0u;
-			// inner nodes base + t and base + t + 512: links and heights when their leaf ranges lie
-			// inside the chunk
-			uint32_t h[2] = { 0u, 0u };
+			// inner nodes base + t and base + t + 512 (0: not all of their leaves are in the chunk)
+			uint32_t w[2] = { 0u, 0u };
 #pragma unroll
 			for (int q = 0; q < 2; q++)
 			{
 				const uint32_t tq = t + q * kChunkThreads, x = base + tq;
 				if (tq < cnt && x < ni)
-				{
-					const uint32_t r = __ldg(node_range + x);
-					if (min(x, r) >= base && max(x, r) < base + cnt)
-					{
-						// children of a node inside the chunk are inside it too (checked, not assumed)
-						const uint2 c = __ldg(children + x);
-						const uint32_t ia = c.x >= ni ? c.x - ni - base : c.x - base, ib = c.y >= ni ? c.y - ni - base : c.y - base;
-						if (ia < cnt && ib < cnt)
-						{
-							s_child[tq] = (ia | (c.x >= ni ? 0x8000u : 0u)) | ((ib | (c.y >= ni ? 0x8000u : 0u)) << 16);
-							h[q] = __ldg(height + x);
-						}
-						else
-							atomicExch(health, 0u);
-					}
-				}
+					w[q] = __ldg(words + x);
 			}
 #pragma unroll
 			for (int q = 0; q < 2; q++)
@@ -631,7 +827,8 @@ namespace u26
 					s_leaf[tq] = sbox(mn, mx);
 				}
 			}
-			const uint32_t wmax = __reduce_max_sync(0xFFFFFFFFu, max(h[0], h[1]));
+			__syncthreads();
+			const uint32_t wmax = __reduce_max_sync(0xFFFFFFFFu, max(w[0], w[1])) >> 22;
 			if ((t & 31) == 0 && wmax)
 				atomicMax(&s_hmax, wmax);
 			__syncthreads();
@@ -641,12 +838,11 @@ namespace u26
 #pragma unroll
 				for (int q = 0; q < 2; q++)
 				{
-					if (h[q] != lv)
+					if (w[q] >> 22 != lv)
 						continue;
-					const uint32_t tq = t + q * kChunkThreads;
-					const uint32_t c = s_child[tq], ca = c & 0xFFFFu, cb = c >> 16;
-					s_inner[tq] = unite_s((ca & 0x8000u) ? s_leaf[ca & 0x3FFu] : s_inner[ca & 0x3FFu],
-						(cb & 0x8000u) ? s_leaf[cb & 0x3FFu] : s_inner[cb & 0x3FFu]);
+					const uint32_t ca = w[q] & 0x7FFu, cb = (w[q] >> 11) & 0x7FFu;
+					// the leaf bit is the slot's place behind the inner boxes' (s_inner follows s_leaf)
+					s_inner[t + q * kChunkThreads] = unite_s(s_leaf[ca ^ 0x400u], s_leaf[cb ^ 0x400u]);
 				}
 				__syncthreads();
 			}
@@ -657,11 +853,12 @@ namespace u26
 				if (tq < cnt)
 				{
 					store_sbox(boxes + ni + base + tq, s_leaf[tq]);
-					if (h[q])
+					if (w[q])
 						store_sbox(boxes + base + tq, s_inner[tq]);
 				}
 			}
-			// the chunk's treelet roots' boxes, also in a compact array for the top-tree launch
+			// the chunk's treelet roots' boxes, also in the compact array that the top-tree launch reads (two per
+			// top node, at the place of the child that they are)
 			if (root_box)
 			{
 				const uint32_t tb0 = chunk_tb[blockIdx.x], tb1 = chunk_tb[blockIdx.x + 1];
@@ -670,96 +867,71 @@ namespace u26
 					const uint32_t x = roots[b];
 					const uint32_t k = x >= ni ? x - ni - base : x - base;
 					if (k < cnt)
-						root_box[b] = x >= ni ? s_leaf[k] : s_inner[k];
+						root_box[root_slot[b]] = x >= ni ? s_leaf[k] : s_inner[k];
 					else
 						atomicExch(health, 0u);
 				}
 			}
 		}
 
-		// The top tree in one block: the treelet roots' boxes are read once, then the top nodes are
-		// united height by height. SHARED (every box fits in shared memory, at most kTopSlots x 1024
-		// top nodes): each thread holds its nodes' links, ids and heights in registers, so a height
-		// step touches shared memory only (its box stores go out behind it). Otherwise the
-		// children are read back through L2 (the block's barrier orders its own stores before the
-		// next height's loads).
-		constexpr uint32_t kTopSlots = 8;
-		template <bool SHARED>
+		// The top tree in one block, height by height. Up to kTopShared top nodes, their boxes and links are in
+		// shared memory: first every node takes its treelet children's boxes (one pass of independent
+		// loads), a height step reads and writes shared memory only, and the boxes go out at the end. Otherwise
+		// boxes and links go through L2 (the block's barrier orders its own stores before the next height's loads).
+		constexpr uint32_t kTopShared = 7u * 1024u;
+		constexpr size_t kTopSmem = (sizeof(SBox) + sizeof(uint2)) * kTopShared;
 		__global__ void __launch_bounds__(1024) refit_top_kernel(NodeBox* __restrict__ boxes, const uint32_t* __restrict__ top_nodes,
-			const uint2* __restrict__ top_links, const uint32_t* __restrict__ height_end, uint32_t m, const uint32_t* __restrict__ roots,
-			uint32_t nt, const uint8_t* __restrict__ top_height, const SBox* __restrict__ root_box, uint32_t* __restrict__ health)
+			const uint2* __restrict__ top_links, const uint32_t* __restrict__ level_end, const uint32_t* __restrict__ info,
+			const SBox* __restrict__ root_box, uint32_t* __restrict__ health)
 		{
-			extern __shared__ SBox s_box[]; // [nt] treelet roots, then [m] top nodes
+			extern __shared__ __align__(16) unsigned char s_raw[];
+			SBox* s_box = reinterpret_cast<SBox*>(s_raw);
+			uint2* s_link = reinterpret_cast<uint2*>(s_box + kTopShared);
+			__shared__ uint32_t s_end[kMaxHeight + 1];
 			const uint32_t t = threadIdx.x;
+			const uint32_t m = info[0], nt = info[1];
+			const bool shared = m <= kTopShared;
 			auto valid = [&](uint32_t id, uint32_t j) { return (id & kTopRoot) ? (id & ~kTopRoot) < nt : id < j; };
-			if constexpr (SHARED)
+			if (t <= kMaxHeight)
+				s_end[t] = min(level_end[t], m);
+			if (shared)
 			{
-				uint2 l[kTopSlots];
-				uint32_t node[kTopSlots], hh[kTopSlots];
-				uint32_t hmax = 0, hmin = kMaxHeight + 1;
-#pragma unroll
-				for (uint32_t k = 0; k < kTopSlots; k++)
+#pragma unroll 4
+				for (uint32_t j = t; j < m; j += 1024u)
 				{
-					const uint32_t j = t + k * blockDim.x;
-					hh[k] = 0;
-					if (j < m)
+					uint2 l = top_links[j];
+					if (!valid(l.x, j) || !valid(l.y, j))
 					{
-						l[k] = top_links[j];
-						node[k] = top_nodes[j];
-						hh[k] = top_height[j];
-						hmax = max(hmax, hh[k]);
-						hmin = min(hmin, hh[k]);
+						// a plan that does not match the tree
+						atomicExch(health, 0u);
+						l = make_uint2(kTopRoot, kTopRoot);
 					}
-				}
-				// the treelet roots' boxes: one coalesced read of the compact copy
-				for (uint32_t b = t; b < nt; b += blockDim.x)
-					s_box[b] = root_box[b];
-				// the heights present: the loop runs from the lowest top node's height to the root's
-				hmax = __reduce_max_sync(0xFFFFFFFFu, hmax);
-				hmin = __reduce_min_sync(0xFFFFFFFFu, hmin);
-				__shared__ uint32_t s_hmax, s_hmin;
-				if (t == 0)
-				{
-					s_hmax = 0;
-					s_hmin = kMaxHeight + 1;
-				}
-				__syncthreads();
-				if ((t & 31) == 0)
-				{
-					atomicMax(&s_hmax, hmax);
-					atomicMin(&s_hmin, hmin);
-				}
-				__syncthreads();
-				hmax = s_hmax;
-				for (uint32_t lv = s_hmin; lv <= hmax; lv++)
-				{
-#pragma unroll
-					for (uint32_t k = 0; k < kTopSlots; k++)
-					{
-						if (hh[k] != lv)
-							continue;
-						const uint32_t j = t + k * blockDim.x;
-						if (!valid(l[k].x, j) || !valid(l[k].y, j))
-						{
-							atomicExch(health, 0u);
-							continue;
-						}
-						const SBox a = (l[k].x & kTopRoot) ? s_box[l[k].x & ~kTopRoot] : s_box[nt + l[k].x];
-						const SBox c = (l[k].y & kTopRoot) ? s_box[l[k].y & ~kTopRoot] : s_box[nt + l[k].y];
-						const SBox u = unite_s(a, c);
-						s_box[nt + j] = u;
-						store_sbox(boxes + node[k], u);
-					}
-					__syncthreads();
+					s_link[j] = l;
+					const bool rx = (l.x & kTopRoot) != 0u, ry = (l.y & kTopRoot) != 0u;
+					if (rx && ry)
+						s_box[j] = unite_s(root_box[2u * j], root_box[2u * j + 1u]);
+					else if (rx || ry)
+						s_box[j] = root_box[2u * j + (rx ? 0u : 1u)];
 				}
 			}
-			else
+			__syncthreads();
+			uint32_t begin = 0;
+			for (uint32_t h = 1; h <= kMaxHeight && begin < m; h++)
 			{
-				uint32_t begin = 0;
-				for (uint32_t h = 1; h <= kMaxHeight && begin < m; h++)
+				const uint32_t end = s_end[h];
+				for (uint32_t j = begin + t; j < end; j += 1024u)
 				{
-					const uint32_t end = max(begin, height_end[h]);
-					for (uint32_t j = begin + t; j < end && j < m; j += blockDim.x)
+					SBox u;
+					if (shared)
+					{
+						const uint2 l = s_link[j];
+						const bool rx = (l.x & kTopRoot) != 0u, ry = (l.y & kTopRoot) != 0u;
+						u = s_box[j];
+						if (!rx || !ry)
+							s_box[j] = unite_s(rx ? u : s_box[l.x], ry ? u : s_box[l.y]);
+						continue;
+					}
+					else
 					{
 						const uint2 l = top_links[j];
 						if (!valid(l.x, j) || !valid(l.y, j))
@@ -767,12 +939,29 @@ namespace u26
 							atomicExch(health, 0u);
 							continue;
 						}
-						auto child = [&](uint32_t id) { return load_box6(boxes + ((id & kTopRoot) ? roots[id & ~kTopRoot] : top_nodes[id])); };
-						store_box6(boxes + top_nodes[j], unite(child(l.x), child(l.y)), 1.0f);
+						auto child = [&](uint32_t id, uint32_t side)
+						{
+							if (id & kTopRoot)
+								return root_box[2u * j + side];
+							const NodeBox* p = boxes + top_nodes[id];
+							const float4 a = __ldcg(&p->mn), b = __ldcg(&p->mx);
+							return sbox(mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z));
+						};
+						u = unite_s(child(l.x, 0u), child(l.y, 1u));
 					}
+					store_sbox(boxes + top_nodes[j], u);
+				}
+				if (end > begin)
+				{
 					begin = end;
 					__syncthreads();
 				}
+			}
+			if (shared)
+			{
+#pragma unroll 4
+				for (uint32_t j = t; j < m; j += 1024u)
+					store_sbox(boxes + top_nodes[j], s_box[j]);
 			}
 		}
 
@@ -878,12 +1067,38 @@ namespace u26
 		U26_CUDA(ctx, t->children.reserve(sizeof(uint2) * nn));
 		U26_CUDA(ctx, t->object_idx.reserve(sizeof(uint32_t) * nn));
 		U26_CUDA(ctx, t->node_aabb.reserve(sizeof(NodeBox) * nn));
-		U26_CUDA(ctx, t->block_aabb.reserve(sizeof(float) * 6 * div_up(n, 256)));
+		U26_CUDA(ctx, t->block_aabb.reserve(sizeof(float) * 6 * kReduceBlocks + sizeof(uint32_t)));
+		U26_CUDA(ctx, cudaMemsetAsync(t->block_aabb.ptr, 0, sizeof(float) * 6 * kReduceBlocks + sizeof(uint32_t), ctx->stream));
 		U26_CUDA(ctx, t->global_aabb.reserve(sizeof(float) * 6));
-		U26_CUDA(ctx, t->refit_flags.reserve(sizeof(uint32_t) * std::max<uint32_t>(n - 1, 1)));
 		U26_CUDA(ctx, t->node_range.reserve(sizeof(uint32_t) * std::max<uint32_t>(n - 1, 1)));
-		U26_CUDA(ctx, t->height.reserve(std::max<uint32_t>(n - 1, 1)));
-		U26_CUDA(ctx, t->height_end.reserve(sizeof(uint32_t) * (kMaxHeight + 1)));
+		const uint32_t cap = plan_capacity(n), chunks = chunk_bound(n), words = div_up(n, 32);
+		// construction scratch in words: head [64], root_bits, top_raw [cap][2], top scratch
+		// (when it does not fit in shared memory), top_list [cap], lo, jump x 2, flag [cap + 1 each]
+		const uint64_t w4 = (words + 3u) & ~3u, c2 = (uint64_t(cap) + 1u) & ~uint64_t(1);
+		const uint64_t scratch = 64u + w4 + 2u * c2 + (cap > kTopScratchShared ? 4u * c2 : 0u) + 5u * uint64_t(cap + 1u);
+		// the refit plan and its scratch: one allocation, every part on a 256-byte boundary
+		struct Part
+		{
+			DevView* view;
+			uint64_t bytes;
+		};
+		const Part parts[] = { { &t->plan_words, sizeof(uint32_t) * uint64_t(std::max<uint32_t>(n - 1, 1)) }, { &t->plan_info, sizeof(uint32_t) * 4 },
+			{ &t->chunk_lo, sizeof(uint32_t) * uint64_t(chunks + 1) }, { &t->chunk_tb, sizeof(uint32_t) * uint64_t(chunks + 1) },
+			{ &t->roots, sizeof(uint32_t) * uint64_t(cap) }, { &t->root_slot, sizeof(uint32_t) * uint64_t(cap) },
+			{ &t->root_box, 2u * sizeof(SBox) * uint64_t(cap) }, { &t->root_height, cap },
+			{ &t->top_nodes, sizeof(uint32_t) * uint64_t(cap) }, { &t->top_links, sizeof(uint2) * uint64_t(cap) },
+			{ &t->level_end, sizeof(uint32_t) * (kMaxHeight + 1) }, { &t->plan_scratch, sizeof(uint32_t) * scratch } };
+		uint64_t total = 0;
+		for (const Part& q : parts)
+			total += (q.bytes + 255u) & ~uint64_t(255);
+		U26_CUDA(ctx, t->plan.reserve(total));
+		total = 0;
+		for (const Part& q : parts)
+		{
+			q.view->ptr = static_cast<unsigned char*>(t->plan.ptr) + total;
+			total += (q.bytes + 255u) & ~uint64_t(255);
+		}
+		U26_CUDA(ctx, cudaMemsetAsync(t->plan_info.ptr, 0, sizeof(uint32_t) * 4, ctx->stream));
 		if (t->type != U26_TREE_VERT)
 			U26_CUDA(ctx, t->leaf_prims.reserve(sizeof(uint32_t) * (t->type == U26_TREE_FACE ? 3u : 2u) * size_t(n)));
 		U26_CUDA(ctx, t->health.reserve(sizeof(uint32_t)));
@@ -943,18 +1158,8 @@ U26_API void u26_lbvh_destroy(u26_lbvh* t)
 	t->node_aabb.release();
 	t->block_aabb.release();
 	t->global_aabb.release();
-	t->refit_flags.release();
 	t->node_range.release();
-	t->height.release();
-	t->chunk_lo.release();
-	t->top_nodes.release();
-	t->top_links.release();
-	t->height_end.release();
-	t->roots.release();
-	t->chunk_tb.release();
-	t->top_height.release();
-	t->root_box.release();
-	t->plan_scratch.release();
+	t->plan.release();
 	t->leaf_prims.release();
 	t->health.release();
 	t->sorter.release();
@@ -966,99 +1171,37 @@ U26_API u26_status u26_lbvh_reduce_aabb(u26_lbvh* t, const float* x, uint32_t nu
 	if (!t || !x || (t->type != U26_TREE_VERT && !prims))
 		return t ? set_error(t->ctx, U26_ERR_INVALID_INPUT, "u26_lbvh_reduce_aabb: null input") : U26_ERR_INVALID_INPUT;
 	u26_ctx* ctx = t->ctx;
+	// lbvh.cpp:999-1021: the edge/face trees reduce ceil(num_verts/256) blocks of 256 primitives in the second pass.
 	const uint32_t nb_leaf = div_up(t->n, 256);
-	// lbvh.cpp:999-1021: the edge/face trees reduce ceil(num_verts/256) blocks in the second pass.
-	uint32_t nb = (t->type == U26_TREE_VERT || t->full_global_aabb) ? nb_leaf : std::min(nb_leaf, div_up(num_verts, 256));
-	if (nb == 0)
-		nb = 1;
-	U26_DISPATCH_TYPE(t->type, reduce_blocks_kernel, nb_leaf, 256, ctx->stream, x, prims, t->n, t->block_aabb.as<float>());
-	U26_TRY(after_launch(ctx, "reduce_blocks_kernel"));
-	reduce_final_kernel<<<1, 256, 0, ctx->stream>>>(t->block_aabb.as<float>(), nb, t->global_aabb.as<float>());
-	U26_TRY(after_launch(ctx, "reduce_final_kernel"));
+	const uint32_t nb = (t->type == U26_TREE_VERT || t->full_global_aabb) ? nb_leaf : std::max(std::min(nb_leaf, div_up(num_verts, 256)), 1u);
+	const uint32_t count = nb == nb_leaf ? t->n : nb * 256u;
+	float* blocks = t->block_aabb.as<float>();
+	U26_DISPATCH_TYPE(t->type, reduce_aabb_kernel, std::min(nb, kReduceBlocks), 256, ctx->stream, x, prims, count, blocks,
+		reinterpret_cast<uint32_t*>(blocks + 6 * kReduceBlocks), t->global_aabb.as<float>());
+	U26_TRY(after_launch(ctx, "reduce_aabb_kernel"));
 	t->last_x = x;
 	t->last_prims = prims;
 	t->last_num_verts = num_verts;
 	return U26_OK;
 }
 
-// The refit plan of a constructed tree (heights, treelets, chunks, top nodes by height).
-static u26_status refit_plan(u26_lbvh* t)
+// The kernels' dynamic shared memory (above the 48 KB default), set once per device.
+static u26_status size_plan_kernels(u26_ctx* ctx)
 {
-	u26_ctx* ctx = t->ctx;
-	cudaStream_t st = ctx->stream;
-	const uint32_t n = t->n, ni = n - 1, nn = 2 * n - 1;
-	uint32_t* health = t->health.as<uint32_t>();
-	// heights
-	U26_CUDA(ctx, cudaMemsetAsync(t->refit_flags.ptr, 0, sizeof(uint32_t) * ni, st));
-	U26_CUDA(ctx, cudaMemsetAsync(t->height.ptr, 0, ni, st));
-	height_kernel<<<div_up(n, 256), 256, 0, st>>>(t->parent.as<uint32_t>(), t->children.as<uint2>(), n, t->refit_flags.as<uint32_t>(),
-		t->height.as<uint8_t>(), health);
-	U26_TRY(after_launch(ctx, "height_kernel"));
-	// scratch: counts[2], top keys / vals [ni], root keys / vals [n], compact map [nn], root sizes [n]
-	// every region starts on a 256-byte boundary
-	auto up = [](size_t v) { return (v + 255) & ~size_t(255); };
-	const size_t off_tk = 256, off_tv = up(off_tk + 8 * size_t(ni)), off_rk = up(off_tv + 4 * size_t(ni)), off_rv = up(off_rk + 8 * size_t(n)),
-				 off_map = up(off_rv + 4 * size_t(n)), off_sz = up(off_map + 4 * size_t(nn)), total = up(off_sz + 4 * size_t(n));
-	U26_CUDA(ctx, t->plan_scratch.reserve(total));
-	unsigned char* sc = static_cast<unsigned char*>(t->plan_scratch.ptr);
-	uint32_t* counts = reinterpret_cast<uint32_t*>(sc);
-	uint64_t* top_keys = reinterpret_cast<uint64_t*>(sc + off_tk);
-	uint32_t* top_vals = reinterpret_cast<uint32_t*>(sc + off_tv);
-	uint64_t* root_keys = reinterpret_cast<uint64_t*>(sc + off_rk);
-	uint32_t* root_vals = reinterpret_cast<uint32_t*>(sc + off_rv);
-	uint32_t* cmap = reinterpret_cast<uint32_t*>(sc + off_map);
-	uint32_t* root_size = reinterpret_cast<uint32_t*>(sc + off_sz);
-	U26_CUDA(ctx, cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), st));
-	treelet_mark_kernel<<<div_up(nn, 256), 256, 0, st>>>(t->parent.as<uint32_t>(), t->node_range.as<uint32_t>(), t->height.as<uint8_t>(), n,
-		counts, top_keys, top_vals, root_keys, root_vals);
-	U26_TRY(after_launch(ctx, "treelet_mark_kernel"));
-	uint32_t mt[2] = { 0, 0 };
-	U26_CUDA(ctx, cudaMemcpyAsync(mt, counts, sizeof(mt), cudaMemcpyDeviceToHost, st));
-	U26_CUDA(ctx, cudaStreamSynchronize(st));
-	const uint32_t m = mt[0], nt = mt[1];
-	if (nt == 0 || nt > n || m > ni)
-		return set_error(ctx, U26_ERR_INVALID_INPUT, "refit plan: %u treelets, %u top nodes for %u leaves", nt, m, n);
-	if (m > 1)
-		U26_TRY(t->sorter.sort(ctx, top_keys, top_vals, m, 0, 40));
-	if (nt > 1)
-		U26_TRY(t->sorter.sort(ctx, root_keys, root_vals, nt, 0, 32));
-	U26_CUDA(ctx, t->top_nodes.reserve(sizeof(uint32_t) * std::max(m, 1u)));
-	U26_CUDA(ctx, t->top_links.reserve(sizeof(uint2) * std::max(m, 1u)));
-	U26_CUDA(ctx, t->roots.reserve(sizeof(uint32_t) * nt));
-	U26_CUDA(ctx, t->chunk_lo.reserve(sizeof(uint32_t) * (nt + 2)));
-	U26_CUDA(ctx, t->chunk_tb.reserve(sizeof(uint32_t) * (nt + 2)));
-	U26_CUDA(ctx, t->top_height.reserve(std::max(m, 1u)));
-	U26_CUDA(ctx, t->root_box.reserve(sizeof(SBox) * nt));
-	if (m)
-		U26_CUDA(ctx, cudaMemcpyAsync(t->top_nodes.ptr, top_vals, sizeof(uint32_t) * m, cudaMemcpyDeviceToDevice, st));
-	U26_CUDA(ctx, cudaMemcpyAsync(t->roots.ptr, root_vals, sizeof(uint32_t) * nt, cudaMemcpyDeviceToDevice, st));
-	treelet_map_kernel<<<div_up(m + nt, 256), 256, 0, st>>>(t->top_nodes.as<uint32_t>(), m, t->roots.as<uint32_t>(), nt, cmap);
-	U26_TRY(after_launch(ctx, "treelet_map_kernel"));
-	U26_CUDA(ctx, cudaMemsetAsync(t->height_end.ptr, 0, sizeof(uint32_t) * (kMaxHeight + 1), st));
-	treelet_links_kernel<<<div_up(std::max(m, nt), 256), 256, 0, st>>>(t->top_nodes.as<uint32_t>(), m, t->children.as<uint2>(), cmap,
-		t->height.as<uint8_t>(), t->top_links.as<uint2>(), t->height_end.as<uint32_t>(), t->roots.as<uint32_t>(), nt,
-		t->node_range.as<uint32_t>(), n, root_size, t->top_height.as<uint8_t>());
-	U26_TRY(after_launch(ctx, "treelet_links_kernel"));
-	treelet_chunks_kernel<<<1, 32, 0, st>>>(root_size, nt, t->chunk_lo.as<uint32_t>(), t->chunk_tb.as<uint32_t>(), counts);
-	U26_TRY(after_launch(ctx, "treelet_chunks_kernel"));
-	U26_CUDA(ctx, cudaMemcpyAsync(mt, counts, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-	U26_CUDA(ctx, cudaStreamSynchronize(st));
-	t->nchunks = mt[0];
-	t->ntop = m;
-	t->ntreelets = nt;
-	const size_t top_bytes = sizeof(SBox) * (size_t(m) + nt);
-	t->top_in_shared = top_bytes <= kTopSharedBytes && m <= kTopSlots * 1024u;
-	if (t->top_in_shared && m)
-		U26_CUDA(ctx, cudaFuncSetAttribute(refit_top_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTopSharedBytes)));
-	// the chunk kernels' dynamic shared memory (above the 48 KB default)
+	static std::atomic<bool> sized[64];
+	const bool known = ctx->device >= 0 && ctx->device < 64;
+	if (known && sized[ctx->device].load(std::memory_order_acquire))
+		return U26_OK;
 	const void* chunk_kernels[] = { (const void*)refit_chunk_kernel<U26_TREE_VERT, false>, (const void*)refit_chunk_kernel<U26_TREE_VERT, true>,
 		(const void*)refit_chunk_kernel<U26_TREE_EDGE, false>, (const void*)refit_chunk_kernel<U26_TREE_EDGE, true>,
 		(const void*)refit_chunk_kernel<U26_TREE_FACE, false>, (const void*)refit_chunk_kernel<U26_TREE_FACE, true> };
 	for (const void* k : chunk_kernels)
 		U26_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kChunkSmem)));
-	// the lists and the compact map (about 40 B per leaf) are needed at construction only; the
-	// stream is idle here (synchronised above)
-	t->plan_scratch.release();
+	U26_CUDA(ctx, cudaFuncSetAttribute(refit_top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTopSmem)));
+	U26_CUDA(ctx, cudaFuncSetAttribute(plan_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(uint32_t) * 4u * kChainShared)));
+	U26_CUDA(ctx, cudaFuncSetAttribute(plan_top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TopScratch) * kTopScratchShared)));
+	if (known)
+		sized[ctx->device].store(true, std::memory_order_release);
 	return U26_OK;
 }
 
@@ -1070,43 +1213,79 @@ U26_API u26_status u26_lbvh_construct_tree(u26_lbvh* t)
 	if (!t->last_x)
 		return set_error(ctx, U26_ERR_INVALID_INPUT, "u26_lbvh_construct_tree: call u26_lbvh_reduce_aabb first");
 	const uint32_t n = t->n;
+	U26_TRY(size_plan_kernels(ctx));
 	uint64_t* keys = t->morton_sorted.as<uint64_t>();
 	uint32_t* vals = t->sorted_get_original.as<uint32_t>();
+	uint32_t* health = t->health.as<uint32_t>();
+	const uint32_t cap = plan_capacity(n), words = div_up(n, 32), w4 = (words + 3u) & ~3u;
+	const uint64_t c2 = (uint64_t(cap) + 1u) & ~uint64_t(1);
+	// the sort's other buffers are free after it
+	U26_CUDA(ctx, t->sorter.keys_alt.reserve(sizeof(uint64_t) * n));
+	U26_CUDA(ctx, t->sorter.vals_alt.reserve(sizeof(uint32_t) * n));
+	uint32_t* sc = t->plan_scratch.as<uint32_t>();
+	auto take = [&](uint64_t count)
+	{
+		uint32_t* p = sc;
+		sc += count;
+		return p;
+	};
+	// (every region up to the top scratch starts on a 16-byte boundary)
+	Plan plan;
+	plan.cap = cap;
+	plan.head = take(64);
+	plan.root_bits = take(w4);
+	plan.root_at = t->sorter.keys_alt.as<uint2>();
+	plan.top_at = t->sorter.vals_alt.as<uint32_t>();
+	TopScratch* top_scratch = cap > kTopScratchShared ? reinterpret_cast<TopScratch*>(take(4u * c2)) : nullptr;
+	plan.top_raw = reinterpret_cast<uint2*>(take(2u * c2));
+	plan.top_list = take(cap);
+	plan.lo = take(cap + 1u);
+	plan.jump[0] = take(cap + 1u);
+	plan.jump[1] = take(cap + 1u);
+	plan.flag = take(cap + 1u);
+	U26_CUDA(ctx, cudaMemsetAsync(plan.head, 0, sizeof(uint32_t) * (64u + w4), ctx->stream));
 	U26_DISPATCH_TYPE(t->type, morton_kernel, div_up(n, 256), 256, ctx->stream, t->last_x, t->last_prims, n,
-		t->global_aabb.as<float>(), keys, vals);
+		t->global_aabb.as<float>(), keys, vals, health);
 	U26_TRY(after_launch(ctx, "morton_kernel"));
 	// Keys are unique and values start as the identity: a stable sort of the Morton bits
 	// [32, 62) reproduces the 64-bit key order.
 	U26_TRY(t->sorter.sort(ctx, keys, vals, n, 32, 62));
-	apply_sorted_kernel<<<div_up(n, 256), 256, 0, ctx->stream>>>(vals, n, t->children.as<uint2>(), t->object_idx.as<uint32_t>(),
-		t->parent.as<uint32_t>(), t->health.as<uint32_t>());
-	U26_TRY(after_launch(ctx, "apply_sorted_kernel"));
-	if (n > 1)
-	{
-		karras_kernel<<<div_up(n - 1, 256), 256, 0, ctx->stream>>>(keys, n, t->children.as<uint2>(), t->parent.as<uint32_t>(),
-			t->node_range.as<uint32_t>());
-		U26_TRY(after_launch(ctx, "karras_kernel"));
-		check_kernel<<<div_up(n - 1, 256), 256, 0, ctx->stream>>>(t->children.as<uint2>(), t->parent.as<uint32_t>(), n - 1,
-			t->health.as<uint32_t>());
-		U26_TRY(after_launch(ctx, "check_kernel"));
-	}
-	// the primitive table in leaf order, for the refits' coalesced leaf reads (the mesh
-	// topology is fixed between constructions; a refit given another table gathers)
+	// (leaf_prims: the mesh topology is fixed between constructions; a refit given another
+	// table gathers)
 	t->leaf_prims_src = nullptr;
+	auto karras = [&](auto* kernel)
+	{
+		kernel<<<div_up(n, 256), 256, 0, ctx->stream>>>(keys, vals, n, t->last_prims, t->leaf_prims.as<uint32_t>(), t->children.as<uint2>(),
+			t->object_idx.as<uint32_t>(), t->parent.as<uint32_t>(), t->node_range.as<uint32_t>(), plan);
+	};
 	if (t->type == U26_TREE_FACE)
-	{
-		permute_prims_kernel<3><<<div_up(n, 256), 256, 0, ctx->stream>>>(vals, t->last_prims, n, t->leaf_prims.as<uint32_t>());
-		U26_TRY(after_launch(ctx, "permute_prims_kernel"));
-		t->leaf_prims_src = t->last_prims;
-	}
+		karras(&karras_kernel<3>);
 	else if (t->type == U26_TREE_EDGE)
-	{
-		permute_prims_kernel<2><<<div_up(n, 256), 256, 0, ctx->stream>>>(vals, t->last_prims, n, t->leaf_prims.as<uint32_t>());
-		U26_TRY(after_launch(ctx, "permute_prims_kernel"));
+		karras(&karras_kernel<2>);
+	else
+		karras(&karras_kernel<0>);
+	U26_TRY(after_launch(ctx, "karras_kernel"));
+	if (t->type != U26_TREE_VERT)
 		t->leaf_prims_src = t->last_prims;
-	}
 	if (n > 1)
-		U26_TRY(refit_plan(t));
+	{
+		uint32_t* info = t->plan_info.as<uint32_t>();
+		const uint32_t chunks = chunk_bound(n);
+		plan_chunks_kernel<<<1, 1024, sizeof(uint32_t) * 4u * std::min(cap + 1u, kChainShared), ctx->stream>>>(plan, n, t->roots.as<uint32_t>(), t->chunk_lo.as<uint32_t>(), t->chunk_tb.as<uint32_t>(),
+			chunks, info, health);
+		U26_TRY(after_launch(ctx, "plan_chunks_kernel"));
+		plan_words_kernel<<<chunks, kChunkThreads, 0, ctx->stream>>>(t->parent.as<uint32_t>(), t->children.as<uint2>(), t->node_range.as<uint32_t>(),
+			n, t->chunk_lo.as<uint32_t>(), t->chunk_tb.as<uint32_t>(), info, t->roots.as<uint32_t>(), t->plan_words.as<uint32_t>(),
+			t->root_height.as<uint8_t>(), health);
+		U26_TRY(after_launch(ctx, "plan_words_kernel"));
+		if (n > kTreelet)
+		{
+			plan_top_kernel<<<1, 1024, sizeof(TopScratch) * std::min(cap, kTopScratchShared), ctx->stream>>>(plan, t->parent.as<uint32_t>(),
+				t->children.as<uint2>(), info, t->root_height.as<uint8_t>(), top_scratch, t->top_nodes.as<uint32_t>(), t->top_links.as<uint2>(),
+				t->root_slot.as<uint32_t>(), t->level_end.as<uint32_t>(), health);
+			U26_TRY(after_launch(ctx, "plan_top_kernel"));
+		}
+	}
 	t->built = true;
 	return U26_OK;
 }
@@ -1135,12 +1314,14 @@ static u26_status refit_impl(u26_lbvh* t, bool fused, const float* thickness, co
 	if (!t->built)
 		return set_error(ctx, U26_ERR_INVALID_INPUT, "refit: call u26_lbvh_construct_tree first");
 	const bool sorted = fused && prims && prims == t->leaf_prims_src;
-	SBox* root_box = (t->ntop && t->top_in_shared) ? t->root_box.as<SBox>() : nullptr;
+	SBox* root_box = t->n > kTreelet ? t->root_box.as<SBox>() : nullptr;
 	const uint32_t* lp = sorted ? t->leaf_prims.as<uint32_t>() : prims;
+	const uint32_t* info = t->plan_info.as<uint32_t>();
+	// (the chunk count stays on the device: blocks past it leave at once)
 #define U26_REFIT(T, F)                                                                                                          \
-	refit_chunk_kernel<T, F><<<t->nchunks, kChunkThreads, kChunkSmem, ctx->stream>>>(t->sorted_get_original.as<uint32_t>(), t->node_aabb.as<NodeBox>(), \
-		x0, x1, thickness, lp, sorted, t->children.as<uint2>(), t->node_range.as<uint32_t>(), t->height.as<uint8_t>(),                  \
-		t->chunk_lo.as<uint32_t>(), t->n, t->chunk_tb.as<uint32_t>(), t->roots.as<uint32_t>(), root_box, t->health.as<uint32_t>())
+	refit_chunk_kernel<T, F><<<chunk_bound(t->n), kChunkThreads, kChunkSmem, ctx->stream>>>(t->sorted_get_original.as<uint32_t>(), \
+		t->node_aabb.as<NodeBox>(), x0, x1, thickness, lp, sorted, t->plan_words.as<uint32_t>(), info, t->chunk_lo.as<uint32_t>(),  \
+		t->n, t->chunk_tb.as<uint32_t>(), t->roots.as<uint32_t>(), t->root_slot.as<uint32_t>(), root_box, t->health.as<uint32_t>())
 	if (t->type == U26_TREE_FACE)
 	{
 		if (fused)
@@ -1161,16 +1342,10 @@ static u26_status refit_impl(u26_lbvh* t, bool fused, const float* thickness, co
 		U26_REFIT(U26_TREE_VERT, false);
 #undef U26_REFIT
 	U26_TRY(after_launch(ctx, "refit_chunk_kernel"));
-	if (t->ntop == 0)
+	if (t->n <= kTreelet)
 		return U26_OK;
-	if (t->top_in_shared)
-		refit_top_kernel<true><<<1, 1024, sizeof(SBox) * (size_t(t->ntop) + t->ntreelets), ctx->stream>>>(t->node_aabb.as<NodeBox>(),
-			t->top_nodes.as<uint32_t>(), t->top_links.as<uint2>(), t->height_end.as<uint32_t>(), t->ntop, t->roots.as<uint32_t>(), t->ntreelets,
-			t->top_height.as<uint8_t>(), t->root_box.as<SBox>(), t->health.as<uint32_t>());
-	else
-		refit_top_kernel<false><<<1, 1024, 0, ctx->stream>>>(t->node_aabb.as<NodeBox>(), t->top_nodes.as<uint32_t>(), t->top_links.as<uint2>(),
-			t->height_end.as<uint32_t>(), t->ntop, t->roots.as<uint32_t>(), t->ntreelets, t->top_height.as<uint8_t>(), nullptr,
-			t->health.as<uint32_t>());
+	refit_top_kernel<<<1, 1024, kTopSmem, ctx->stream>>>(t->node_aabb.as<NodeBox>(), t->top_nodes.as<uint32_t>(), t->top_links.as<uint2>(),
+		t->level_end.as<uint32_t>(), info, t->root_box.as<SBox>(), t->health.as<uint32_t>());
 	return after_launch(ctx, "refit_top_kernel");
 }
 

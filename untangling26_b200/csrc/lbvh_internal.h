@@ -3,6 +3,17 @@
 #pragma once
 #include "u26_internal.h"
 
+namespace u26
+{
+	// A part of a DevBuf.
+	struct DevView
+	{
+		void* ptr = nullptr;
+		template <typename T>
+		T* as() const { return static_cast<T*>(ptr); }
+	};
+} // namespace u26
+
 struct u26_lbvh
 {
 	u26_ctx* ctx = nullptr;
@@ -14,23 +25,24 @@ struct u26_lbvh
 	u26::DevBuf children;			 // uint32[2n-1][2]
 	u26::DevBuf object_idx;			 // uint32[2n-1]
 	u26::DevBuf node_aabb;			 // NodeBox[2n-1]
-	u26::DevBuf block_aabb;			 // float[ceil(n/256)][6]
+	u26::DevBuf block_aabb;			 // float[blocks][6] of the global AABB's reduction, then its arrival count
 	u26::DevBuf global_aabb;		 // float[6]
-	u26::DevBuf refit_flags;		 // uint32[max(n-1,1)]: arrival counters of the height pass (construction)
 	u26::DevBuf node_range;			 // uint32[max(n-1,1)]: inner node i covers leaves [min(i, r), max(i, r)], r = node_range[i]
-	// refit plan, prepared by construct_tree (one per topology)
-	u26::DevBuf height;			 // uint8[max(n-1,1)]: inner node height (leaves 0)
-	u26::DevBuf chunk_lo;		 // uint32[nchunks + 1]: first leaf of each refit chunk, then n
-	u26::DevBuf top_nodes;		 // uint32[m]: nodes of more than 1024 leaves, by height
-	u26::DevBuf top_links;		 // uint2[m]: their children as compact ids (top j, or 0x80000000 | treelet b)
-	u26::DevBuf height_end;		 // uint32[65]: end of each height's run in top_nodes (0: none)
-	u26::DevBuf roots;			 // uint32[nt]: treelet roots (maximal subtrees of <= 1024 leaves) in leaf order
-	u26::DevBuf chunk_tb;		 // uint32[nchunks + 1]: first treelet of each chunk, then nt
-	u26::DevBuf top_height;		 // uint8[m]: heights of top_nodes
-	u26::DevBuf root_box;		 // float[nt][6]: the treelet roots' boxes of the last refit, compact
-	u26::DevBuf plan_scratch;	 // construction scratch (list keys, counts, compact map), freed when the plan is made
-	uint32_t nchunks = 0, ntop = 0, ntreelets = 0;
-	bool top_in_shared = false;
+	// refit plan, prepared by construct_tree (one per topology; its counts stay on the device): parts of one
+	// allocation
+	u26::DevBuf plan;
+	u26::DevView plan_info;		 // uint32[4]: top nodes m, treelets nt, chunks
+	u26::DevView plan_words;		 // uint32[max(n-1,1)]: chunk-local child slots and height of each inner node
+	u26::DevView chunk_lo;		 // uint32[chunks + 1]: first leaf of each refit chunk, then n
+	u26::DevView chunk_tb;		 // uint32[chunks + 1]: first treelet of each chunk, then nt
+	u26::DevView roots;			 // uint32[nt]: treelet roots (maximal subtrees of <= 1024 leaves) in leaf order
+	u26::DevView root_height;	 // uint8[nt]: their heights
+	u26::DevView root_slot;		 // uint32[nt]: 2 x the parent's place in top_nodes + the side
+	u26::DevView root_box;		 // float[2m][6]: their boxes of the last refit, by root_slot
+	u26::DevView top_nodes;		 // uint32[m]: nodes of more than 1024 leaves, by height
+	u26::DevView top_links;		 // uint2[m]: their children as compact ids (top j, or 0x80000000 | treelet b)
+	u26::DevView level_end;		 // uint32[65]: end of each height's run in top_nodes
+	u26::DevView plan_scratch;	 // construction scratch (about 2 B per leaf)
 	u26::DevBuf leaf_prims;			 // uint32[n][K]: the primitive table in leaf order (edge / face trees)
 	const uint32_t* leaf_prims_src = nullptr; // the table leaf_prims was permuted from
 	u26::DevBuf health;				 // uint32[1]: 1 healthy
