@@ -197,7 +197,7 @@ class Workload:
             # one batch of 32 contours per pass: the 199 contours of the first pass grow to whole
             # sheets (4.9 G requests, 75 s per pass); the traversal configuration is the batch
             # workload's tuned one (tuning here would run 18 full ray-casting passes)
-            self.params = dict(max_contours=32, batch_size=32, autotune=0, raycast_config=2)
+            self.params = dict(max_contours=32, batch_size=32, autotune=0, raycast_config=11)
             self.repair = True
             # the fixed step: a quarter of the assembled response, so that no vertex moves more
             # than 0.375 mm (a pair asks for up to the 3 mm response depth, half per side) between
@@ -209,7 +209,7 @@ class Workload:
             self.config = {"workload": "layered_sheets_5x512x512", "seed": 4, "layers": 5, "triangles": int(self.full.num_faces),
                            "spacing_mm": 1, "displacement_mm": "U[2, 20] multi-octave", "directions": "reference seeds (<=10)",
                            "opt_iterations": 0, "contours": "first 32 of each pass (one batch)", "update": "response step, scale 0.25",
-                           "raycast_config": "fixed 4x7"}
+                           "raycast_config": "fixed 4x5q"}
         else:
             raise SystemExit(f"unknown workload {name}")
         self.config["l2"] = "flushed between steps (256 MB write)"
@@ -470,7 +470,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-full-batch", action="store_true", help="skip the whole-batch chosen / plain timing")
     ap.add_argument("--raycast-config", default=None,
-                    help="a fixed traversal configuration ('4x7', '8x7q', ...) instead of the autotuner's choice")
+                    help="a fixed traversal configuration ('4x5', '8x5q', ...) instead of the autotuner's choice")
     ap.add_argument("--profile-pass", action="store_true",
                     help="for ncu (--profile-from-start off): warm-up passes, then one pass of the timed workload "
                          "inside cudaProfilerStart / Stop; prints one line and exits")

@@ -848,14 +848,9 @@ namespace u26
 
 		// one counter atomic per group of lanes emitting together (slot order does not matter:
 		// hit keys are unique and sorted afterwards)
-		__device__ __forceinline__ void emit(const HitSink& hs, uint32_t task, uint32_t type, uint32_t src, uint32_t dst, float b0, float b1,
-			float dist)
+		__device__ __forceinline__ void store_hit(const HitSink& hs, uint32_t slot, uint32_t task, uint32_t type, uint32_t src, uint32_t dst,
+			float b0, float b1, float dist)
 		{
-			cg::coalesced_group g = cg::coalesced_threads();
-			uint32_t base = 0;
-			if (g.thread_rank() == 0)
-				base = atomicAdd(hs.count, g.size());
-			const uint32_t slot = g.shfl(base, 0) + g.thread_rank();
 			if (slot >= hs.cap)
 				return;
 			const uint64_t key = (uint64_t(task) << (2 + 2 * hs.b)) | (uint64_t(type) << (2 * hs.b)) | (uint64_t(src) << hs.b) | uint64_t(dst);
@@ -864,6 +859,15 @@ namespace u26
 			hs.payload[3 * slot] = b0;
 			hs.payload[3 * slot + 1] = b1;
 			hs.payload[3 * slot + 2] = dist;
+		}
+		__device__ __forceinline__ void emit(const HitSink& hs, uint32_t task, uint32_t type, uint32_t src, uint32_t dst, float b0, float b1,
+			float dist)
+		{
+			cg::coalesced_group g = cg::coalesced_threads();
+			uint32_t base = 0;
+			if (g.thread_rank() == 0)
+				base = atomicAdd(hs.count, g.size());
+			store_hit(hs, g.shfl(base, 0) + g.thread_rank(), task, type, src, dst, b0, b1, dist);
 		}
 
 		// FP64 rechecks (predicates.cuh) of one VF / FV ray - triangle test and one swept edge -
@@ -885,33 +889,311 @@ namespace u26
 			return 1u | (h64 != hit32 ? 2u : 0u);
 		}
 
-		// Packet traversal: a warp takes 32 consecutive requests (one task's candidate vertices
-		// or edges in BFS order: one direction, nearby origins) and walks the union of their
-		// paths with one shared stack, every lane testing its own ray against each popped node
-		// (one broadcast load per node) and its own leaf primitives. Face-tree requests (VF,
-		// FV) and edge-tree requests (EE) of a warp take one packet walk each. The grid is
+		// Ray traversal: a warp takes 32 consecutive requests (one task's candidate vertices or edges in Morton
+		// order: one direction, nearby origins), every lane walks its own ray or swept edge with a stack of its
+		// own, and the leaves met go into a queue in shared memory as (primitive, lane) entries, from which
+		// full batches of 32 are tested. The leaf work (candidate bit, triangle or edge gather, exact test, error
+		// band) is most of the instructions, and its lanes are all busy that way; a step loads both
+		// children's boxes at once and goes on with one of them in registers. Face-tree requests (VF,
+		// FV) and edge-tree requests (EE) of a warp take one walk each. The grid is
 		// `split` parts x the requests rounded up to warps; part p starts at the p-th node of the
 		// target tree's frontier for that split, so every (ray, leaf) pair is decided once.
 		// MINB: resident 128-thread blocks per SM the registers are sized for.
+		// Bound by the latency of the divergent node loads (a third of the issue slots wait for them). 64.5 M
+		// requests of 16 two-body scenes (161 node and 28 leaf tests each): 225 ms with the warp walking the union
+		// of its requests' paths and testing a leaf with the lanes that met it (three times the nodes, 19 of 32
+		// lanes busy), 113 ms now; two 64 x 64 sheets 14.3 ms, 6.3 ms; folded 64 x 64 sheet, 26 directions, 19.0
+		// ms, 11.4 ms.
 		constexpr int kStack = 64;
+		struct RayWarp
+		{
+			float f[14][32];	  // a ray's or swept edge's constants, by lane
+			uint32_t u[8][32];
+			uint32_t prim[128]; // leaf queue: 31 left over + 2 x 32 new entries at most
+			uint8_t from[128];
+		};
+		__device__ __forceinline__ NodeBox load_node(const NodeBox* p)
+		{
+			// one 32-byte load (nodes start on 32-byte boundaries)
+			NodeBox b;
+			asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+				: "=f"(b.mn.x), "=f"(b.mn.y), "=f"(b.mn.z), "=f"(b.mn.w), "=f"(b.mx.x), "=f"(b.mx.y), "=f"(b.mx.z), "=f"(b.mx.w)
+				: "l"(p));
+			return b;
+		}
+		// What the leaf tests read, and where the hits go.
+		struct LeafArgs
+		{
+			const float* x;
+			const uint2* edges;
+			const uint32_t* faces;
+			const uint32_t *bits_e, *bits_f;
+			uint32_t e_words, f_words; // bitmap words per slot
+			HitSink sink;
+		};
+		extern __shared__ __align__(16) unsigned char s_ray_raw[]; // RayWarp per warp
+		__device__ __forceinline__ RayWarp& ray_warp() { return reinterpret_cast<RayWarp*>(s_ray_raw)[threadIdx.x >> 5]; }
+
+		// 32 leaf tests, entry (primitive, lane) k < n in lane k. Out of line: one call per 32 tests, and the walk
+		// keeps its registers. Returns 1 when the entry's primitive is a candidate, plus its FP64 recheck (256) and
+		// flip (65536).
+		template <bool RECHECK>
+		__device__ __noinline__ uint32_t test_triangles(const LeafArgs& L, uint32_t fid, uint32_t from, uint32_t n)
+		{
+			const RayWarp& W = ray_warp();
+			const uint32_t lane = threadIdx.x & 31u;
+			uint32_t told = 0;
+			const uint32_t flags = W.u[5][from], v = W.u[0][from];
+			bool hit32 = false;
+			f3 bary = mk3(0.0f);
+			float tt = 0.0f;
+			if (lane < n &&
+				bit_test(L.bits_f + size_t(W.u[2][from]) * L.f_words, W.u[3][from], W.u[4][from], fid))
+			{
+				told = 1u;
+				const uint32_t f0 = __ldg(L.faces + 3 * fid), f1 = __ldg(L.faces + 3 * fid + 1), f2 = __ldg(L.faces + 3 * fid + 2);
+				if (v != f0 && v != f1 && v != f2 && (flags & 2u))
+				{
+					const f3 o = mk3(W.f[0][from], W.f[1][from], W.f[2][from]), sr = mk3(W.f[3][from], W.f[4][from], W.f[5][from]);
+					const float len = W.f[9][from];
+					const f3 A = ld3(L.x, f0), B = ld3(L.x, f1), C = ld3(L.x, f2);
+					if (ray_tri(o, sr, len, A, B, C, tt, bary))
+					{
+						tt = tt * W.f[10][from];
+						hit32 = tt >= 0.0f && tt <= 1.0f;
+					}
+					if (RECHECK && tri_needs_recheck(o, sr, len, A, B, C))
+					{
+						const uint32_t rc = recheck_vf(o, mk3(W.f[6][from], W.f[7][from], W.f[8][from]), A, B, C, hit32);
+						told += (rc & 1u) << 8;
+						told += (rc >> 1) << 16;
+					}
+				}
+			}
+			const uint32_t m = __ballot_sync(0xFFFFFFFFu, hit32);
+			if (m)
+			{
+				uint32_t base = 0;
+				if (lane == 0)
+					base = atomicAdd(L.sink.count, uint32_t(__popc(m)));
+				base = __shfl_sync(0xFFFFFFFFu, base, 0);
+				const bool f = flags & 1u;
+				if (hit32)
+					store_hit(L.sink, base + __popc(m & ((1u << lane) - 1u)), W.u[1][from], f ? 2u : 0u, f ? fid : v, f ? v : fid, bary.x,
+						bary.y, tt * 1.0f);
+			}
+			return told;
+		}
+		template <bool RECHECK>
+		__device__ __noinline__ uint32_t test_edges(const LeafArgs& L, uint32_t e2, uint32_t from, uint32_t n)
+		{
+			const RayWarp& W = ray_warp();
+			const uint32_t lane = threadIdx.x & 31u;
+			uint32_t told = 0;
+			bool ee_hit = false;
+			float t1 = 0.0f, t2 = 0.0f, sv = 0.0f;
+			if (lane < n &&
+				bit_test(L.bits_e + size_t(W.u[2][from]) * L.e_words, W.u[3][from], W.u[4][from], e2))
+			{
+				told = 1u;
+				const uint2 qv = __ldg(L.edges + e2);
+				const uint32_t ex = W.u[6][from], ey = W.u[7][from];
+				if (!(ex == qv.x || ex == qv.y || ey == qv.x || ey == qv.y))
+				{
+					const f3 q0 = ld3(L.x, qv.x), q1 = ld3(L.x, qv.y);
+					const f3 p0 = mk3(W.f[0][from], W.f[1][from], W.f[2][from]), e1 = mk3(W.f[3][from], W.f[4][from], W.f[5][from]);
+					const f3 dir = mk3(W.f[6][from], W.f[7][from], W.f[8][from]), pn = mk3(W.f[9][from], W.f[10][from], W.f[11][from]);
+					const float pd = W.f[12][from], ray_max = W.f[13][from];
+					const bool plane = W.u[5][from] != 0u;
+					bool sep = false;
+					if (plane)
+					{
+						const float d0 = dot(pn, q0) - pd;
+						const float d1 = dot(pn, q1) - pd;
+						sep = (d0 > 1e-6f && d1 > 1e-6f) || (d0 < -1e-6f && d1 < -1e-6f);
+					}
+					if (!sep)
+					{
+						const f3 e2v = q1 - q0;
+						const f3 rr = q0 - p0;
+						const f3 nn = cross(e1, e2v);
+						const float det = -dot(dir, nn);
+						if (!(fabsf(det) < 1e-10f))
+						{
+							// x = n_x / det. Misses decided before the division, only where the test
+							// below rejects too: a numerator (|n| >= 1e-20, so n / det stays nonzero) of
+							// the other sign than det, or t1, t2 beyond 1 / sv beyond ray_max by a 1e-5
+							// relative margin; each numerator is computed once the earlier ones pass
+							const float n_sv = -dot(rr, cross(e1, e2v));
+							const float adet = fabsf(det);
+							const bool screen = adet <= 1e20f;
+							auto neg = [&](float v)
+							{ return fabsf(v) >= 1e-20f && ((v > 0.0f) != (det > 0.0f)); };
+							const float lim = adet * (1.0f + 1e-5f);
+							bool maybe = !(screen && (neg(n_sv) || (ray_max >= 1e-20f && fabsf(n_sv) > lim * ray_max)));
+							float n_t1 = 0.0f, n_t2 = 0.0f;
+							if (maybe)
+							{
+								n_t1 = -dot(dir, cross(rr, e2v));
+								maybe = !(screen && (neg(n_t1) || fabsf(n_t1) > lim));
+							}
+							if (maybe)
+							{
+								n_t2 = dot(dir, cross(e1, rr));
+								maybe = !(screen && (neg(n_t2) || fabsf(n_t2) > lim));
+							}
+							if (maybe)
+							{
+								const float inv = 1.0f / det;
+								sv = n_sv * inv;
+								t1 = n_t1 * inv;
+								t2 = n_t2 * inv;
+								ee_hit = sv >= 0.0f && sv <= ray_max && t1 >= 0.0f && t1 <= 1.0f && t2 >= 0.0f && t2 <= 1.0f;
+							}
+						}
+					}
+					Band bd;
+					if (RECHECK)
+						edge_edge_band(p0, e1, dir, ray_max, plane, pn, pd, q0, q1, bd);
+					if (RECHECK && bd.recheck())
+					{
+						const uint32_t rc = recheck_ee(p0, e1, dir, ray_max, q0, q1, ee_hit);
+						told += (rc & 1u) << 8;
+						told += (rc >> 1) << 16;
+					}
+				}
+			}
+			const uint32_t m = __ballot_sync(0xFFFFFFFFu, ee_hit);
+			if (m)
+			{
+				uint32_t base = 0;
+				if (lane == 0)
+					base = atomicAdd(L.sink.count, uint32_t(__popc(m)));
+				base = __shfl_sync(0xFFFFFFFFu, base, 0);
+				if (ee_hit)
+					store_hit(L.sink, base + __popc(m & ((1u << lane) - 1u)), W.u[1][from], 1u, W.u[0][from], e2, 1.0f - t1, 1.0f - t2, sv);
+			}
+			return told;
+		}
+
+		// One walk of a warp: meets(box) decides a node for this lane's ray; flush(prim, lane, n) takes n queue
+		// entries, one per lane (all lanes call it). visited: boxes this lane tested, leaves: leaves it met.
+		template <class Meets, class Flush>
+		__device__ __forceinline__ void ray_walk(RayWarp& W, const NodeBox* __restrict__ nodes, uint32_t start, uint32_t& visited, uint32_t& leaves,
+			uint32_t* __restrict__ dev_err, Meets meets, Flush flush)
+		{
+			constexpr uint32_t kAll = 0xFFFFFFFFu;
+			const uint32_t lane = threadIdx.x & 31u;
+			uint32_t count = 0;
+			auto push_leaf = [&](bool hit, uint32_t prim)
+			{
+				const uint32_t m = __ballot_sync(kAll, hit);
+				if (hit)
+				{
+					const uint32_t k = count + __popc(m & ((1u << lane) - 1u));
+					W.prim[k] = prim;
+					W.from[k] = uint8_t(lane);
+					leaves++;
+				}
+				count += __popc(m);
+			};
+			auto drain = [&](uint32_t keep)
+			{
+				__syncwarp();
+				while (count > keep)
+				{
+					const uint32_t n = min(count, 32u);
+					count -= n;
+					const uint32_t k = count + min(lane, n - 1u);
+					flush(W.prim[k], uint32_t(W.from[k]), n);
+				}
+				__syncwarp();
+			};
+			uint2 cur = make_uint2(0u, 0u); // the children of the inner node that the lane stands at
+			bool on = start != kInvalid;
+			{
+				bool leaf = false;
+				if (on)
+				{
+					const NodeBox b = load_node(nodes + start);
+					visited++;
+					cur = make_uint2(__float_as_uint(b.mn.w), __float_as_uint(b.mx.w));
+					on = meets(b);
+					leaf = on && cur.y == kInvalid;
+				}
+				push_leaf(leaf, cur.x);
+				on = on && !leaf;
+			}
+			uint2 stack[kStack];
+			uint32_t top = 0, loop = 0;
+			while (__any_sync(kAll, on))
+			{
+				bool hx = false, hy = false;
+				uint2 nx = cur, ny = cur;
+				if (on)
+				{
+					const NodeBox bx = load_node(nodes + cur.x), by = load_node(nodes + cur.y);
+					visited += 2u;
+					hx = meets(bx);
+					hy = meets(by);
+					nx = make_uint2(__float_as_uint(bx.mn.w), __float_as_uint(bx.mx.w));
+					ny = make_uint2(__float_as_uint(by.mn.w), __float_as_uint(by.mx.w));
+				}
+				const bool leaf_x = nx.y == kInvalid, leaf_y = ny.y == kInvalid;
+				push_leaf(hx && leaf_x, nx.x);
+				push_leaf(hy && leaf_y, ny.x);
+				const bool go_x = hx && !leaf_x, go_y = hy && !leaf_y;
+				if (go_x && go_y)
+				{
+					if (top < uint32_t(kStack))
+						stack[top++] = ny;
+					else
+					{
+						atomicOr(dev_err, U26_DEVERR_STACK_OVERFLOW);
+						on = false;
+					}
+				}
+				if (go_x)
+					cur = nx;
+				else if (go_y)
+					cur = ny;
+				else if (top > 0u)
+					cur = stack[--top];
+				else
+					on = false;
+				if (++loop > 4000000u)
+				{
+					if (on)
+						atomicOr(dev_err, U26_DEVERR_ITERATION_CAP);
+					on = false;
+				}
+				if (count >= 64u)
+					drain(31u);
+			}
+			drain(0u);
+		}
+
 		template <bool RECHECK, int MINB, bool QUEUE>
 		__global__ void __launch_bounds__(128, MINB) raycast_kernel(const Task* __restrict__ tasks, uint32_t ntasks, uint32_t total,
 			const Slot* __restrict__ slots, const uint32_t* __restrict__ cand_v, const uint32_t* __restrict__ cand_e, uint32_t v_stride,
-			uint32_t e_stride, uint32_t f_stride, const uint32_t* __restrict__ bits_e, const uint32_t* __restrict__ bits_f,
-			const NodeBox* __restrict__ fgrow, const NodeBox* __restrict__ egrow, const uint32_t* __restrict__ ffront,
-			const uint32_t* __restrict__ efront, const float* __restrict__ x, const uint2* __restrict__ edges,
-			const uint32_t* __restrict__ faces, const float* __restrict__ slot_box, HitSink sink, unsigned long long* __restrict__ stats,
-			uint32_t split, uint32_t* __restrict__ queue, uint32_t* __restrict__ dev_err)
+			uint32_t e_stride, const NodeBox* __restrict__ fgrow, const NodeBox* __restrict__ egrow, const uint32_t* __restrict__ ffront,
+			const uint32_t* __restrict__ efront, const float* __restrict__ slot_box, const __grid_constant__ LeafArgs L,
+			unsigned long long* __restrict__ stats, uint32_t split, uint32_t* __restrict__ queue, uint32_t* __restrict__ dev_err)
 		{
+			const float* __restrict__ x = L.x;
+			const uint2* __restrict__ edges = L.edges;
+			RayWarp& W = ray_warp();
 			const int lane = threadIdx.x & 31;
-			// the packet's traversal stack lives in registers across the warp: entry k in lane k & 31
-			// of s_lo (k < 32) or s_hi (k >= 32); every lane holds the same stack pointer
-			uint32_t s_lo = 0u, s_hi = 0u;
 			const uint32_t warps_per_part = (total + 31u) >> 5;
-			const uint32_t items = split * warps_per_part; // (part, packet) work items
-			uint32_t tested = 0, visited = 0, etested = 0, ctested = 0, rechecks = 0, flips = 0, reqs = 0;
-			uint32_t fetch_nodes = 0, fetch_tris = 0, fetch_edges = 0; // warp-uniform: data each packet brings in
-			uint32_t ray_visits = 0; // the node tests this ray alone would make: its start + 2 per inner node it enters
+			const uint32_t items = split * warps_per_part; // (part, 32 requests) work items
+			uint32_t tested = 0, visited = 0, etested = 0, ctested = 0, rechecks = 0, flips = 0, reqs = 0, told = 0;
+			auto count_told = [&]()
+			{
+				ctested += told & 0xFFu;
+				rechecks += (told >> 8) & 0xFFu;
+				flips += told >> 16;
+				told = 0u;
+			};
 			// QUEUE (persistent form): every warp takes work items from a device counter until none is
 			// left, so no warp idles while the other warps of its block finish; otherwise the grid
 			// has one warp per item
@@ -936,8 +1218,7 @@ namespace u26
 			int kind = 0; // 1: VF / FV ray on the face tree, 2: EE swept edge on the edge tree
 			uint32_t t = 0, vid = 0, eid = 0, tobj = 0;
 			bool fv = false;
-			const uint32_t* bits = nullptr;
-			uint32_t tgt_lo = 0, tgt_cnt = 0;
+			uint32_t tgt_slot = 0, tgt_lo = 0, tgt_cnt = 0;
 			f3 dir = mk3(0.0f), orig = mk3(0.0f), sray = mk3(0.0f);
 			float slen = 0.0f, inv_len = 0.0f, t_lo = 0.0f, t_hi = 1.0f;
 			bool seg_ok = false;
@@ -971,7 +1252,7 @@ namespace u26
 					tgt_lo = tgt.f_lo;
 					tgt_cnt = tgt.f_cnt;
 					tobj = tgt.pad[1];
-					bits = bits_f + size_t(fv ? tk.slot0 : tk.slot1) * (f_stride / 32 + 1);
+					tgt_slot = fv ? tk.slot0 : tk.slot1;
 					const f3 cast = fv ? -dir : dir;
 					orig = ld3(x, vid);
 					const f3 end = orig + cast * 1.0f;
@@ -992,7 +1273,7 @@ namespace u26
 				{
 					// EE: swept edge of side 0 along dir onto edges of side 1
 					eid = cand_e[size_t(tk.slot0) * e_stride + (local - tk.n_vf)];
-					bits = bits_e + size_t(tk.slot1) * (e_stride / 32 + 1);
+					tgt_slot = tk.slot1;
 					const Slot s1 = slots[tk.slot1];
 					tgt_lo = s1.e_lo;
 					tgt_cnt = s1.e_cnt;
@@ -1004,103 +1285,23 @@ namespace u26
 				}
 			}
 
-			// ---- face tree: VF / FV rays of the warp
-			// each lane starts at its target object's subtree root of this part; lanes with the
-			// same start walk together
+			// ---- face tree: VF / FV rays of the warp, each from its target object's subtree root of this
+			// part
 			const uint32_t foff = front_offset(split);
-			const uint32_t fstart_l = kind == 1 ? ffront[size_t(tobj) * kFrontStride + foff + part] : kInvalid;
-			uint32_t fpending = __ballot_sync(0xFFFFFFFFu, fstart_l != kInvalid);
-			while (fpending != 0u)
+			const uint32_t fstart = kind == 1 ? ffront[size_t(tobj) * kFrontStride + foff + part] : kInvalid;
+			if (__any_sync(0xFFFFFFFFu, fstart != kInvalid))
 			{
-				const uint32_t fstart = __shfl_sync(0xFFFFFFFFu, fstart_l, __ffs(fpending) - 1);
-				const bool on = fstart_l == fstart;
-				fpending &= ~__ballot_sync(0xFFFFFFFFu, on);
-				ray_visits += on ? 1u : 0u;
-				// depth first: a hit inner node continues with its first child and stacks the second
-				uint32_t node = fstart;
-				int sp = 0;
-				uint32_t loop = 0;
-				for (;;)
-				{
-					NodeBox b;
-					b.mn = __ldg(&fgrow[node].mn);
-					b.mx = __ldg(&fgrow[node].mx);
-					visited += on ? 1u : 0u;
-					fetch_nodes++;
-					const bool hit = on && ray_grown_box(slab, t_lo, t_hi, b);
-					const uint32_t link_a = __float_as_uint(b.mn.w), link_b = __float_as_uint(b.mx.w);
-					bool descend = false;
-					if (__ballot_sync(0xFFFFFFFFu, hit) == 0u)
-					{
-					}
-					else if (link_b == kInvalid)
-					{
-						const uint32_t fid = link_a;
-						fetch_tris++;
-						if (hit)
-						{
-							tested++;
-							if (bit_test(bits, tgt_lo, tgt_cnt, fid))
-							{
-								ctested++;
-								const uint32_t f0 = faces[3 * fid], f1 = faces[3 * fid + 1], f2 = faces[3 * fid + 2];
-								if (vid != f0 && vid != f1 && vid != f2 && seg_ok)
-								{
-									f3 bary;
-									float tt;
-									const f3 A = ld3(x, f0), B = ld3(x, f1), C = ld3(x, f2);
-									bool hit32 = false;
-									if (ray_tri(orig, sray, slen, A, B, C, tt, bary))
-									{
-										tt = tt * inv_len;
-										hit32 = tt >= 0.0f && tt <= 1.0f;
-										if (hit32)
-											emit(sink, t, fv ? 2u : 0u, fv ? fid : vid, fv ? vid : fid, bary.x, bary.y, tt * 1.0f);
-									}
-									if (RECHECK && tri_needs_recheck(orig, sray, slen, A, B, C))
-									{
-										const uint32_t rc = recheck_vf(orig, fv ? -dir : dir, A, B, C, hit32);
-										rechecks += rc & 1u;
-										flips += rc >> 1;
-									}
-								}
-							}
-						}
-						__syncwarp();
-					}
-					else
-					{
-						ray_visits += hit ? 2u : 0u;
-						if (sp + 1 > kStack)
-						{
-							if (lane == 0)
-								atomicOr(dev_err, U26_DEVERR_STACK_OVERFLOW);
-							break;
-						}
-						if (lane == (sp & 31))
-						{
-							if (sp < 32)
-								s_lo = link_b;
-							else
-								s_hi = link_b;
-						}
-						sp++;
-						node = link_a;
-						descend = true;
-					}
-					if (++loop > 4000000u)
-					{
-						if (lane == 0)
-							atomicOr(dev_err, U26_DEVERR_ITERATION_CAP);
-						break;
-					}
-					if (descend)
-						continue;
-					if (sp == 0)
-						break;
-					sp--;
-					node = __shfl_sync(0xFFFFFFFFu, sp < 32 ? s_lo : s_hi, sp & 31);
-				}
+				const f3 cast = fv ? -dir : dir;
+				W.f[0][lane] = orig.x, W.f[1][lane] = orig.y, W.f[2][lane] = orig.z;
+				W.f[3][lane] = sray.x, W.f[4][lane] = sray.y, W.f[5][lane] = sray.z;
+				W.f[6][lane] = cast.x, W.f[7][lane] = cast.y, W.f[8][lane] = cast.z;
+				W.f[9][lane] = slen, W.f[10][lane] = inv_len;
+				W.u[0][lane] = vid, W.u[1][lane] = t, W.u[2][lane] = tgt_slot, W.u[3][lane] = tgt_lo, W.u[4][lane] = tgt_cnt;
+				W.u[5][lane] = (fv ? 1u : 0u) | (seg_ok ? 2u : 0u);
+				__syncwarp();
+				ray_walk(
+					W, fgrow, fstart, visited, tested, dev_err, [&](const NodeBox& b) { return ray_grown_box(slab, t_lo, t_hi, b); },
+					[&](uint32_t fid, uint32_t from, uint32_t n) { told += test_triangles<RECHECK>(L, fid, from, n); count_told(); });
 				__syncwarp();
 			}
 
@@ -1152,163 +1353,47 @@ namespace u26
 						kind = 2;
 				}
 			}
-			const uint32_t estart_l = kind == 2 ? efront[size_t(tobj) * kFrontStride + foff + part] : kInvalid;
-			uint32_t epending = __ballot_sync(0xFFFFFFFFu, estart_l != kInvalid);
-			while (epending != 0u)
+			const uint32_t estart = kind == 2 ? efront[size_t(tobj) * kFrontStride + foff + part] : kInvalid;
+			if (__any_sync(0xFFFFFFFFu, estart != kInvalid))
 			{
-				const uint32_t estart = __shfl_sync(0xFFFFFFFFu, estart_l, __ffs(epending) - 1);
-				const bool on = estart_l == estart;
-				epending &= ~__ballot_sync(0xFFFFFFFFu, on);
-				ray_visits += on ? 1u : 0u;
-				uint32_t node = estart;
-				int sp = 0;
-				uint32_t loop = 0;
-				for (;;)
-				{
-					NodeBox g;
-					g.mn = __ldg(&egrow[node].mn);
-					g.mx = __ldg(&egrow[node].mx);
-					visited += on ? 1u : 0u;
-					fetch_nodes++;
-					bool hit = on && (smn.x <= g.mx.x) & (smx.x >= g.mn.x) & (smn.y <= g.mx.y) & (smx.y >= g.mn.y) & (smn.z <= g.mx.z) &
-						(smx.z >= g.mn.z);
-					// the swept edge lies in the plane (pn, pd): a box that keeps clear of the slab
-					// |dot(pn, q) - pd| <= 1e-6 holds only edges the leaf's separating-plane test
-					// rejects (cached_bvh.cpp:433-473 prunes its nodes the same way). The boxes carry
-					// the 1e-5 (1 + |c|) margin, far above the rounding of this test, so no edge the
-					// leaf test keeps is pruned.
-					// and a box whose extent along dir misses the swept edge's holds no edge it reaches
-					if (hit)
+				W.f[0][lane] = p0.x, W.f[1][lane] = p0.y, W.f[2][lane] = p0.z;
+				W.f[3][lane] = e1.x, W.f[4][lane] = e1.y, W.f[5][lane] = e1.z;
+				W.f[6][lane] = dir.x, W.f[7][lane] = dir.y, W.f[8][lane] = dir.z;
+				W.f[9][lane] = pn.x, W.f[10][lane] = pn.y, W.f[11][lane] = pn.z;
+				W.f[12][lane] = pd, W.f[13][lane] = ray_max;
+				W.u[0][lane] = eid, W.u[1][lane] = t, W.u[2][lane] = tgt_slot, W.u[3][lane] = tgt_lo, W.u[4][lane] = tgt_cnt;
+				W.u[5][lane] = plane ? 1u : 0u, W.u[6][lane] = ev.x, W.u[7][lane] = ev.y;
+				__syncwarp();
+				const uint32_t tested0 = tested;
+				ray_walk(
+					W, egrow, estart, visited, tested, dev_err,
+					[&](const NodeBox& g)
 					{
-						const f3 c = mk3(0.5f * (g.mn.x + g.mx.x), 0.5f * (g.mn.y + g.mx.y), 0.5f * (g.mn.z + g.mx.z));
-						const f3 h = mk3(0.5f * (g.mx.x - g.mn.x), 0.5f * (g.mx.y - g.mn.y), 0.5f * (g.mx.z - g.mn.z));
-						const float cp = dot(c, dir);
-						const float pr = (h.x * fabsf(dir.x) + h.y * fabsf(dir.y)) + h.z * fabsf(dir.z);
-						hit = !(cp + pr < proj_lo || cp - pr > proj_hi);
-						if (hit && plane)
-						{
-							const float rad = (h.x * fabsf(pn.x) + h.y * fabsf(pn.y)) + h.z * fabsf(pn.z);
-							hit = fabsf(dot(pn, c) - pd) <= rad + 1e-6f;
-						}
-					}
-					const uint32_t link_a = __float_as_uint(g.mn.w), link_b = __float_as_uint(g.mx.w);
-					bool descend = false;
-					if (__ballot_sync(0xFFFFFFFFu, hit) == 0u)
-					{
-					}
-					else if (link_b == kInvalid)
-					{
-						const uint32_t e2 = link_a;
-						fetch_edges++;
+						bool hit = (smn.x <= g.mx.x) & (smx.x >= g.mn.x) & (smn.y <= g.mx.y) & (smx.y >= g.mn.y) & (smn.z <= g.mx.z) &
+							(smx.z >= g.mn.z);
+						// the swept edge lies in the plane (pn, pd): a box that keeps clear of the slab
+						// |dot(pn, q) - pd| <= 1e-6 holds only edges the leaf's separating-plane test
+						// rejects (cached_bvh.cpp:433-473 prunes its nodes the same way). The boxes carry
+						// the 1e-5 (1 + |c|) margin, far above the rounding of this test, so no edge the
+						// leaf test keeps is pruned.
+						// and a box whose extent along dir misses the swept edge's holds no edge it reaches
 						if (hit)
 						{
-							tested++;
-							etested++;
-							if (bit_test(bits, tgt_lo, tgt_cnt, e2))
+							const f3 c = mk3(0.5f * (g.mn.x + g.mx.x), 0.5f * (g.mn.y + g.mx.y), 0.5f * (g.mn.z + g.mx.z));
+							const f3 h = mk3(0.5f * (g.mx.x - g.mn.x), 0.5f * (g.mx.y - g.mn.y), 0.5f * (g.mx.z - g.mn.z));
+							const float cp = dot(c, dir);
+							const float pr = (h.x * fabsf(dir.x) + h.y * fabsf(dir.y)) + h.z * fabsf(dir.z);
+							hit = !(cp + pr < proj_lo || cp - pr > proj_hi);
+							if (hit && plane)
 							{
-								ctested++;
-								const uint2 qv = edges[e2];
-								if (!(ev.x == qv.x || ev.x == qv.y || ev.y == qv.x || ev.y == qv.y))
-								{
-									const f3 q0 = ld3(x, qv.x), q1 = ld3(x, qv.y);
-									bool sep = false, ee_hit = false;
-									if (plane)
-									{
-										const float d0 = dot(pn, q0) - pd;
-										const float d1 = dot(pn, q1) - pd;
-										sep = (d0 > 1e-6f && d1 > 1e-6f) || (d0 < -1e-6f && d1 < -1e-6f);
-									}
-									if (!sep)
-									{
-										const f3 e2v = q1 - q0;
-										const f3 rr = q0 - p0;
-										const f3 n = cross(e1, e2v);
-										const float det = -dot(dir, n);
-										if (!(fabsf(det) < 1e-10f))
-										{
-											// x = n_x / det. Misses decided before the division, only where the test
-											// below rejects too: a numerator (|n| >= 1e-20, so n / det stays nonzero) of
-											// the other sign than det, or t1, t2 beyond 1 / sv beyond ray_max by a 1e-5
-											// relative margin; each numerator is computed once the earlier ones pass
-											const float n_sv = -dot(rr, cross(e1, e2v));
-											const float adet = fabsf(det);
-											const bool screen = adet <= 1e20f;
-											auto neg = [&](float v)
-											{ return fabsf(v) >= 1e-20f && ((v > 0.0f) != (det > 0.0f)); };
-											const float lim = adet * (1.0f + 1e-5f);
-											bool maybe = !(screen && (neg(n_sv) || (ray_max >= 1e-20f && fabsf(n_sv) > lim * ray_max)));
-											float n_t1 = 0.0f, n_t2 = 0.0f;
-											if (maybe)
-											{
-												n_t1 = -dot(dir, cross(rr, e2v));
-												maybe = !(screen && (neg(n_t1) || fabsf(n_t1) > lim));
-											}
-											if (maybe)
-											{
-												n_t2 = dot(dir, cross(e1, rr));
-												maybe = !(screen && (neg(n_t2) || fabsf(n_t2) > lim));
-											}
-											if (maybe)
-											{
-												const float inv = 1.0f / det;
-												const float sv = n_sv * inv;
-												const float t1 = n_t1 * inv;
-												const float t2 = n_t2 * inv;
-												if (sv >= 0.0f && sv <= ray_max && t1 >= 0.0f && t1 <= 1.0f && t2 >= 0.0f && t2 <= 1.0f)
-												{
-													ee_hit = true;
-													emit(sink, t, 1u, eid, e2, 1.0f - t1, 1.0f - t2, sv);
-												}
-											}
-										}
-									}
-									Band bd;
-									if (RECHECK)
-										edge_edge_band(p0, e1, dir, ray_max, plane, pn, pd, q0, q1, bd);
-									if (RECHECK && bd.recheck())
-									{
-										const uint32_t rc = recheck_ee(p0, e1, dir, ray_max, q0, q1, ee_hit);
-										rechecks += rc & 1u;
-										flips += rc >> 1;
-									}
-								}
+								const float rad = (h.x * fabsf(pn.x) + h.y * fabsf(pn.y)) + h.z * fabsf(pn.z);
+								hit = fabsf(dot(pn, c) - pd) <= rad + 1e-6f;
 							}
 						}
-						__syncwarp();
-					}
-					else
-					{
-						ray_visits += hit ? 2u : 0u;
-						if (sp + 1 > kStack)
-						{
-							if (lane == 0)
-								atomicOr(dev_err, U26_DEVERR_STACK_OVERFLOW);
-							break;
-						}
-						if (lane == (sp & 31))
-						{
-							if (sp < 32)
-								s_lo = link_b;
-							else
-								s_hi = link_b;
-						}
-						sp++;
-						node = link_a;
-						descend = true;
-					}
-					if (++loop > 4000000u)
-					{
-						if (lane == 0)
-							atomicOr(dev_err, U26_DEVERR_ITERATION_CAP);
-						break;
-					}
-					if (descend)
-						continue;
-					if (sp == 0)
-						break;
-					sp--;
-					node = __shfl_sync(0xFFFFFFFFu, sp < 32 ? s_lo : s_hi, sp & 31);
-				}
+						return hit;
+					},
+					[&](uint32_t e2, uint32_t from, uint32_t n) { told += test_edges<RECHECK>(L, e2, from, n); count_told(); });
+				etested += tested - tested0;
 				__syncwarp();
 			}
 			if constexpr (!QUEUE)
@@ -1320,16 +1405,15 @@ namespace u26
 				const uint32_t rsum = __reduce_add_sync(0xFFFFFFFFu, reqs);
 				const uint32_t vsum = __reduce_add_sync(0xFFFFFFFFu, visited);
 				const uint32_t esum = __reduce_add_sync(0xFFFFFFFFu, etested);
-				const uint32_t rvsum = __reduce_add_sync(0xFFFFFFFFu, ray_visits);
 				const uint32_t csum = __reduce_add_sync(0xFFFFFFFFu, ctested);
 				const uint32_t rcsum = __reduce_add_sync(0xFFFFFFFFu, rechecks);
 				const uint32_t flsum = __reduce_add_sync(0xFFFFFFFFu, flips);
 				if (lane == 0)
 				{
 					// [0] leaf primitive tests, [1] requests, [2] ray-node tests, [3] edge leaf tests,
-					// [4] node fetches, [5] triangle fetches, [6] edge fetches (per packet),
-					// [7] single-ray node visits, [8] leaf tests of candidate targets
-					atomicAdd(stats + 7, (unsigned long long)rvsum);
+					// [4] node fetches, [5] triangle fetches, [6] edge fetches (a ray's walk fetches what it
+					// tests), [7] single-ray node visits, [8] leaf tests of candidate targets
+					atomicAdd(stats + 7, (unsigned long long)vsum);
 					atomicAdd(stats + 8, (unsigned long long)csum);
 					// [9] FP64 rechecks of leaf tests inside their error band, [10] FP32 / FP64 flips
 					if (rcsum)
@@ -1340,32 +1424,37 @@ namespace u26
 					atomicAdd(stats + 1, (unsigned long long)rsum);
 					atomicAdd(stats + 2, (unsigned long long)vsum);
 					atomicAdd(stats + 3, (unsigned long long)esum);
-					atomicAdd(stats + 4, (unsigned long long)fetch_nodes);
-					atomicAdd(stats + 5, (unsigned long long)fetch_tris);
-					atomicAdd(stats + 6, (unsigned long long)fetch_edges);
+					atomicAdd(stats + 4, (unsigned long long)vsum);
+					atomicAdd(stats + 5, (unsigned long long)(tsum - esum));
+					atomicAdd(stats + 6, (unsigned long long)esum);
 				}
 			}
 		}
 
 		// The traversal configurations the autotuner chooses from: subtree parts per request
-		// (4, 8, 16) x resident blocks of 128 threads per SM the registers are sized for (6, 7, 8:
-		// at most 80, 72 or 64 registers per thread) x the grid form (one warp per work item, or a
-		// persistent grid of warps taking items from a queue). The packet is the warp (32 requests).
+		// (4, 8, 16) x resident blocks of 128 threads per SM the registers are sized for (4, 5, 6:
+		// at most 128, 96 or 80 registers per thread) x the grid form (one warp per work item, or a
+		// persistent grid of warps taking items from a queue: the counters go out once per warp and not once
+		// per item). A work item is 32 requests.
 		struct RaycastConfig
 		{
 			uint32_t split;
 			int min_blocks;
 			bool queue;
 		};
-		constexpr RaycastConfig kRaycastConfigs[] = { { 4, 6, false }, { 4, 7, false }, { 4, 8, false }, { 8, 6, false }, { 8, 7, false },
-			{ 8, 8, false }, { 16, 6, false }, { 16, 7, false }, { 16, 8, false }, { 4, 6, true }, { 4, 7, true }, { 4, 8, true }, { 8, 6, true },
-			{ 8, 7, true }, { 8, 8, true }, { 16, 6, true }, { 16, 7, true }, { 16, 8, true } };
-		constexpr int kNumRaycastConfigs = 18, kDefaultRaycastConfig = 4; // 8 parts, 7 blocks per SM, a warp per item
-		using RaycastFn = decltype(&raycast_kernel<false, 7, false>);
+		constexpr RaycastConfig kRaycastConfigs[] = { { 4, 4, false }, { 4, 5, false }, { 4, 6, false }, { 8, 4, false }, { 8, 5, false },
+			{ 8, 6, false }, { 16, 4, false }, { 16, 5, false }, { 16, 6, false }, { 4, 4, true }, { 4, 5, true }, { 4, 6, true }, { 8, 4, true },
+			{ 8, 5, true }, { 8, 6, true }, { 16, 4, true }, { 16, 5, true }, { 16, 6, true } };
+		// The default: the queue at 5 blocks per SM, in 8 parts. Parts share a ray's setup but not its balance: 16
+		// scenes of 2k-60k triangles take 113 ms in 4 parts, 121 in 8; a folded sheet with 26 directions 13.4, 11.4
+		// (10.5 in 16); two 64 x 64 sheets 6.3, 6.8. Launches of kManyRequests and more (the first kind) use 4.
+		constexpr int kNumRaycastConfigs = 18, kDefaultRaycastConfig = 13;
+		constexpr uint32_t kManyRequests = 1u << 20;
+		using RaycastFn = decltype(&raycast_kernel<false, 5, false>);
 		template <bool R, bool Q>
 		inline RaycastFn raycast_variant_q(int min_blocks)
 		{
-			return min_blocks == 6 ? &raycast_kernel<R, 6, Q> : min_blocks == 8 ? &raycast_kernel<R, 8, Q> : &raycast_kernel<R, 7, Q>;
+			return min_blocks == 4 ? &raycast_kernel<R, 4, Q> : min_blocks == 6 ? &raycast_kernel<R, 6, Q> : &raycast_kernel<R, 5, Q>;
 		}
 		inline RaycastFn raycast_variant(bool recheck, int min_blocks, bool queue)
 		{
@@ -4520,6 +4609,7 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 	const bool forced = P->raycast_config >= 1 && P->raycast_config <= uint32_t(kNumRaycastConfigs);
 	const bool tuning = !forced && P->autotune && P->form == 0 && S->tuned_cfg < 0;
 	const int cfg_now = forced ? int(P->raycast_config) - 1 : S->tuned_cfg >= 0 ? S->tuned_cfg : kDefaultRaycastConfig;
+	const bool chosen_by_size = !forced && !tuning && S->tuned_cfg < 0;
 	std::vector<cudaEvent_t> tune_ev;
 	struct EventsGuard
 	{
@@ -4674,7 +4764,9 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 				const bool rc = attempt == 0 && !hits_out && P->fp64_recheck;
 				auto launch = [&](int cfg, unsigned long long* stats) -> u26_status
 				{
-					const RaycastConfig c = kRaycastConfigs[cfg];
+					RaycastConfig c = kRaycastConfigs[cfg];
+					if (chosen_by_size && total_req >= kManyRequests)
+						c.split = 4;
 					const uint64_t nthreads = uint64_t(div_up(total_req, 32u)) * 32u * c.split;
 					uint64_t blocks = div_up64(nthreads, 128);
 					if (c.queue)
@@ -4684,11 +4776,12 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 						U26_CUDA(ctx, cudaMemsetAsync(S->d_queue.ptr, 0, sizeof(uint32_t), st));
 					}
 					const RaycastFn kern = raycast_variant(rc, c.min_blocks, c.queue);
-					kern<<<uint32_t(blocks), 128, 0, st>>>(S->d_tasks.as<Task>(), nt, total_req, S->d_slots.as<Slot>(),
-						S->d_cand_v.as<uint32_t>(), S->d_cand_e.as<uint32_t>(), vs, es_, fs, S->d_bits_e.as<uint32_t>(),
-						S->d_bits_f.as<uint32_t>(), S->d_fgrow.as<NodeBox>(), S->d_egrow.as<NodeBox>(), S->d_front.as<uint32_t>(),
-						S->d_front.as<uint32_t>() + size_t(nobj) * kFrontStride, d_x, S->d_edges.as<uint2>(), S->d_faces.as<uint32_t>(),
-						S->d_slot_box.as<float>(), sink, stats, c.split, S->d_queue.as<uint32_t>(), ctx->dev_err);
+					const LeafArgs leaf{ d_x, S->d_edges.as<uint2>(), S->d_faces.as<uint32_t>(), S->d_bits_e.as<uint32_t>(),
+						S->d_bits_f.as<uint32_t>(), es_ / 32u + 1u, fs / 32u + 1u, sink };
+					kern<<<uint32_t(blocks), 128, 4 * sizeof(RayWarp), st>>>(S->d_tasks.as<Task>(), nt, total_req, S->d_slots.as<Slot>(),
+						S->d_cand_v.as<uint32_t>(), S->d_cand_e.as<uint32_t>(), vs, es_, S->d_fgrow.as<NodeBox>(), S->d_egrow.as<NodeBox>(),
+						S->d_front.as<uint32_t>(), S->d_front.as<uint32_t>() + size_t(nobj) * kFrontStride, S->d_slot_box.as<float>(), leaf,
+						stats, c.split, S->d_queue.as<uint32_t>(), ctx->dev_err);
 					return after_launch(ctx, "raycast_kernel");
 				};
 				if (tuning && attempt == 0 && !hits_out)

@@ -81,9 +81,9 @@ class PrpOutputView(ctypes.Structure):
     ]
 
 # (subtree parts, blocks / SM, persistent work-queue grid)
-RAYCAST_CONFIGS = tuple((p, b, q) for q in (False, True) for p in (4, 8, 16) for b in (6, 7, 8))
+RAYCAST_CONFIGS = tuple((p, b, q) for q in (False, True) for p in (4, 8, 16) for b in (4, 5, 6))
 def config_name(c):
-    """'8x7' (parts x blocks per SM, a warp per item) or '8x7q' (persistent work-queue grid)."""
+    """'8x5' (parts x blocks per SM, a warp per item) or '8x5q' (persistent work-queue grid)."""
     return f"{c[0]}x{c[1]}" + ("q" if c[2] else "")
 
 
