@@ -190,78 +190,116 @@ namespace u26
 		};
 
 		// ------------------------------------------------------------ distances
-		// One CTA per slot. hop/geo/order/mark are slot-strided (stride = largest object).
-		__global__ void __launch_bounds__(256) distances_kernel(Slot* __restrict__ slots, const uint32_t* __restrict__ slot_ids,
+		// Two CTAs per slot: hop distances (BFS) and rest-geodesic distances, which do not depend on each other.
+		// hop/geo/order/mark are slot-strided (stride = largest object). SHARED: the state that the rounds
+		// touch with atomics lives in shared memory (a visited bit per vertex for the BFS; the distance and
+		// a queued bit for the relaxation: 4.125 B per vertex, up to kSharedVerts vertices); otherwise
+		// in global memory. Bound by the rounds' dependent accesses (45 BFS levels and about as many
+		// relaxation rounds on a 64 x 64 sheet): 0.95 ms with one
+		// 256-thread CTA and L2 atomics, 0.29 ms.
+		constexpr uint32_t kDistThreads = 512;
+		constexpr uint32_t kSharedVerts = 53000; // 218,625 bytes
+		inline size_t dist_smem(uint32_t verts) { return 4u * size_t(verts) + 4u * size_t(verts / 32u + 1u); }
+		template <bool SHARED>
+		__global__ void __launch_bounds__(kDistThreads) distances_kernel(Slot* __restrict__ slots, const uint32_t* __restrict__ slot_ids,
 			const uint32_t* __restrict__ bnd, const uint32_t* __restrict__ vav_off, const uint32_t* __restrict__ vav,
 			const float* __restrict__ rest_x, uint32_t stride, uint32_t* __restrict__ hop, float* __restrict__ geo,
 			uint32_t* __restrict__ order, uint32_t* __restrict__ level_end, uint32_t* __restrict__ work, uint32_t* __restrict__ mark,
 			uint32_t* __restrict__ dev_err)
 		{
-			const uint32_t s = slot_ids[blockIdx.x];
-			Slot sl = slots[s];
+			extern __shared__ __align__(16) uint32_t s_dist[];
+			__shared__ uint32_t s_tail, s_n;
+			const uint32_t s = slot_ids[blockIdx.x >> 1];
+			const Slot sl = slots[s];
 			const uint32_t lo = sl.v_lo, cnt = sl.v_cnt;
-			uint32_t* hs = hop + size_t(s) * stride;
-			float* gs = geo + size_t(s) * stride;
-			uint32_t* os = order + size_t(s) * stride;
-			uint32_t* ms = mark + size_t(s) * stride;
-			uint32_t* le = level_end + size_t(s) * (stride + 1);
+			if ((blockIdx.x & 1u) == 0u)
+			{
+				uint32_t* hs = hop + size_t(s) * stride;
+				uint32_t* os = order + size_t(s) * stride;
+				uint32_t* le = level_end + size_t(s) * (stride + 1);
+				for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x)
+					hs[i] = kInf;
+				if (SHARED)
+					for (uint32_t i = threadIdx.x; i < cnt / 32u + 1u; i += blockDim.x)
+						s_dist[i] = 0u;
+				__syncthreads();
+				for (uint32_t j = threadIdx.x; j < sl.bnd_cnt; j += blockDim.x)
+				{
+					// the host only forms slots whose anchors lie in the side's object
+					const uint32_t v = min(bnd[sl.bnd_off + j] - lo, cnt - 1u);
+					hs[v] = 0u;
+					os[j] = v;
+					if (SHARED)
+						atomicOr(s_dist + (v >> 5), 1u << (v & 31u));
+				}
+				if (threadIdx.x == 0)
+				{
+					s_tail = sl.bnd_cnt;
+					le[0] = sl.bnd_cnt;
+				}
+				__syncthreads();
+				// the order array is the queue; level_end[h] = #vertices with hop <= h
+				uint32_t head = 0, tail = sl.bnd_cnt, level = 0;
+				while (head < tail)
+				{
+					for (uint32_t i = head + threadIdx.x; i < tail; i += blockDim.x)
+					{
+						const uint32_t gv = lo + os[i];
+						for (uint32_t k = vav_off[gv]; k < vav_off[gv + 1]; k++)
+						{
+							const uint32_t a = vav[k];
+							if (a < lo || a >= lo + cnt)
+								continue;
+							const uint32_t v = a - lo;
+							bool first;
+							if (SHARED)
+							{
+								const uint32_t bit = 1u << (v & 31u);
+								first = (s_dist[v >> 5] & bit) == 0u && (atomicOr(s_dist + (v >> 5), bit) & bit) == 0u;
+								if (first)
+									hs[v] = level + 1u;
+							}
+							else
+								first = atomicCAS(hs + v, kInf, level + 1u) == kInf;
+							if (first)
+								os[atomicAdd(&s_tail, 1u)] = v;
+						}
+					}
+					__syncthreads();
+					head = tail;
+					tail = s_tail;
+					level++;
+					if (threadIdx.x == 0)
+						le[level] = tail;
+					__syncthreads();
+				}
+				if (threadIdx.x == 0)
+					slots[s].diam = level > 0 && sl.bnd_cnt != 0 ? level - 1u : 0u;
+				return;
+			}
+			// rest-geodesic distance: worklist relaxation to the least fixpoint
 			uint32_t* wa = work + size_t(s) * 2 * stride;
 			uint32_t* wb = wa + stride;
-			__shared__ uint32_t s_tail, s_n;
+			float* out = geo + size_t(s) * stride;
+			uint32_t* gs = SHARED ? s_dist : reinterpret_cast<uint32_t*>(out); // distances as bits (non-negative: ordered alike)
+			uint32_t* queued = SHARED ? s_dist + cnt : mark + size_t(s) * stride; // a bit, or a word, per vertex
 			for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x)
 			{
-				hs[i] = kInf;
-				gs[i] = kGeoInf;
-				ms[i] = 0u;
+				gs[i] = __float_as_uint(kGeoInf);
+				if (!SHARED)
+					queued[i] = 0u;
 			}
+			if (SHARED)
+				for (uint32_t i = threadIdx.x; i < cnt / 32u + 1u; i += blockDim.x)
+					queued[i] = 0u;
 			__syncthreads();
 			for (uint32_t j = threadIdx.x; j < sl.bnd_cnt; j += blockDim.x)
 			{
-				// the host only forms slots whose anchors lie in the side's object
 				const uint32_t v = min(bnd[sl.bnd_off + j] - lo, cnt - 1u);
-				hs[v] = 0u;
-				gs[v] = 0.0f;
-				os[j] = v;
+				gs[v] = 0u;
 				wa[j] = v;
 			}
-			if (threadIdx.x == 0)
-			{
-				s_tail = sl.bnd_cnt;
-				le[0] = sl.bnd_cnt;
-			}
 			__syncthreads();
-			// BFS: the order array is the queue; level_end[h] = #vertices with hop <= h
-			uint32_t head = 0, tail = sl.bnd_cnt, level = 0;
-			while (head < tail)
-			{
-				for (uint32_t i = head + threadIdx.x; i < tail; i += blockDim.x)
-				{
-					const uint32_t v = os[i];
-					const uint32_t gv = lo + v;
-					for (uint32_t k = vav_off[gv]; k < vav_off[gv + 1]; k++)
-					{
-						const uint32_t a = vav[k];
-						if (a < lo || a >= lo + cnt)
-							continue;
-						if (atomicCAS(hs + (a - lo), kInf, level + 1u) == kInf)
-							os[atomicAdd(&s_tail, 1u)] = a - lo;
-					}
-				}
-				__syncthreads();
-				head = tail;
-				tail = s_tail;
-				level++;
-				if (threadIdx.x == 0)
-					le[level] = tail;
-				__syncthreads();
-			}
-			if (threadIdx.x == 0)
-			{
-				slots[s].diam = level > 0 ? level - 1u : 0u;
-				if (sl.bnd_cnt == 0)
-					slots[s].diam = 0u;
-			}
-			// rest-geodesic distance: worklist relaxation to the least fixpoint
 			uint32_t ncur = sl.bnd_cnt;
 			uint32_t* cur = wa;
 			uint32_t* nxt = wb;
@@ -276,28 +314,45 @@ namespace u26
 				{
 					const uint32_t v = cur[i];
 					const uint32_t gv = lo + v;
-					const float d = __uint_as_float(atomicAdd(reinterpret_cast<uint32_t*>(gs + v), 0u));
+					const float d = __uint_as_float(SHARED ? *(volatile uint32_t*)(gs + v) : atomicAdd(gs + v, 0u));
 					const f3 pv = ld3(rest_x, gv);
 					for (uint32_t k = vav_off[gv]; k < vav_off[gv + 1]; k++)
 					{
 						const uint32_t a = vav[k];
 						if (a < lo || a >= lo + cnt)
 							continue;
-						const float nd = d + length(pv - ld3(rest_x, a));
-						const uint32_t nb = __float_as_uint(nd);
-						const uint32_t old = atomicMin(reinterpret_cast<uint32_t*>(gs + (a - lo)), nb);
-						if (nb < old && atomicExch(ms + (a - lo), 1u) == 0u)
-							nxt[atomicAdd(&s_n, 1u)] = a - lo;
+						const uint32_t w = a - lo;
+						const uint32_t nb = __float_as_uint(d + length(pv - ld3(rest_x, a)));
+						if (SHARED && *(volatile uint32_t*)(gs + w) <= nb)
+							continue;
+						if (nb >= atomicMin(gs + w, nb))
+							continue;
+						bool first;
+						if (SHARED)
+						{
+							const uint32_t bit = 1u << (w & 31u);
+							first = (atomicOr(queued + (w >> 5), bit) & bit) == 0u;
+						}
+						else
+							first = atomicExch(queued + w, 1u) == 0u;
+						if (first)
+							nxt[atomicAdd(&s_n, 1u)] = w;
 					}
 				}
 				__syncthreads();
 				const uint32_t nn = s_n;
 				for (uint32_t i = threadIdx.x; i < nn; i += blockDim.x)
-					ms[nxt[i]] = 0u;
+				{
+					const uint32_t w = nxt[i];
+					if (SHARED)
+						queued[w >> 5] = 0u; // (every queued vertex is in the list)
+					else
+						queued[w] = 0u;
+				}
 				__syncthreads();
-				uint32_t* t = cur;
+				uint32_t* x = cur;
 				cur = nxt;
-				nxt = t;
+				nxt = x;
 				ncur = nn;
 				if (++rounds > max_rounds)
 				{
@@ -305,6 +360,12 @@ namespace u26
 						atomicOr(dev_err, U26_DEVERR_ITERATION_CAP);
 					break;
 				}
+			}
+			if (SHARED)
+			{
+				__syncthreads();
+				for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x)
+					out[i] = __uint_as_float(gs[i]);
 			}
 		}
 
@@ -429,7 +490,8 @@ namespace u26
 			}
 		}
 
-		__global__ void __launch_bounds__(256) candidates_kernel(const Slot* __restrict__ slots, const uint32_t* __restrict__ slot_ids,
+		constexpr uint32_t kCandThreads = 1024; // a CTA per slot, bound by its dependent gathers: 133 us with 256, 81 us
+		__global__ void __launch_bounds__(kCandThreads) candidates_kernel(const Slot* __restrict__ slots, const uint32_t* __restrict__ slot_ids,
 			const uint32_t* __restrict__ bnd, const float* __restrict__ x, const uint2* __restrict__ edges,
 			const uint32_t* __restrict__ faces, const uint32_t* __restrict__ vae_off, const uint32_t* __restrict__ vae,
 			const uint32_t* __restrict__ vaf_off, const uint32_t* __restrict__ vaf, uint32_t v_stride, uint32_t e_stride,
@@ -534,7 +596,7 @@ namespace u26
 				}
 			}
 			// block min / max of the candidate boxes
-			__shared__ float red[12][8];
+			__shared__ float red[12][kCandThreads / 32];
 			float v12[12] = { fmn.x, fmn.y, fmn.z, fmx.x, fmx.y, fmx.z, emn.x, emn.y, emn.z, emx.x, emx.y, emx.z };
 			const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -556,7 +618,7 @@ namespace u26
 				const int q = threadIdx.x;
 				const bool is_min = (q % 6) < 3;
 				float v = red[q][0];
-				for (int w = 1; w < 8; w++)
+				for (int w = 1; w < int(kCandThreads / 32); w++)
 					v = is_min ? fminf(v, red[q][w]) : fmaxf(v, red[q][w]);
 				slot_box[12 * size_t(s) + q] = v;
 			}
@@ -2280,6 +2342,21 @@ namespace u26
 			return lo < r.e && ek[lo] == key;
 		}
 
+		// the first entry of a sorted run after those equal to ek[i] (a vertex has an entry per hit, in few
+		// components: doubling steps, then a binary search)
+		__device__ __forceinline__ uint32_t skip_equal(const uint64_t* __restrict__ ek, uint32_t i, uint32_t end)
+		{
+			const uint64_t k = ek[i];
+			uint32_t step = 1;
+			while (end - i > step && ek[i + step] == k)
+			{
+				i += step;
+				step <<= 1;
+			}
+			// ek[i] == k, and i + step is past the equal entries or the run
+			return i + 1u + lower_bound64(ek + i + 1u, min(step, end - i) - 1u, k + 1u);
+		}
+
 		// EF-anchor coverage counted per anchor (prp_fill_combo_eval_info, intersection_
 		// resolver2.cpp:1806-1881): one thread per (task, anchor); every boundary-attached
 		// component that holds a vertex of the anchor's edge on side m and a vertex of its face
@@ -2326,9 +2403,15 @@ namespace u26
 			{
 				uint32_t rl;
 				if (i1 >= E1.e || (i0 < E0.e && (ekeys[i0] & rmask) <= (ekeys[i1] & rmask)))
-					rl = uint32_t(ekeys[i0++] & rmask);
+				{
+					rl = uint32_t(ekeys[i0] & rmask);
+					i0 = skip_equal(ekeys, i0, E0.e);
+				}
 				else
-					rl = uint32_t(ekeys[i1++] & rmask);
+				{
+					rl = uint32_t(ekeys[i1] & rmask);
+					i1 = skip_equal(ekeys, i1, E1.e);
+				}
 				if (rl == last)
 					continue;
 				last = rl;
@@ -2978,80 +3061,61 @@ namespace u26
 			out[t] = o;
 		}
 
-		// The selected support of each listed task in canonical (key) order: one CTA per task
-		// compacts the hits of its best component out of the task's sorted segment.
+		// The selected support of each listed task in canonical (key) order: kCaptureBlocks blocks per task copy the
+		// hits of its best component to their places (the scanned positions of sel_terms_kernel).
+		constexpr uint32_t kCaptureBlocks = 16;
 		__global__ void __launch_bounds__(256) capture_kernel(const uint32_t* __restrict__ list, const uint32_t* __restrict__ out_off,
 			const uint64_t* __restrict__ keys, const uint32_t* __restrict__ root, const uint32_t* __restrict__ best,
-			const uint32_t* __restrict__ seg, const float* __restrict__ pay, HitKeyCodec cd, const uint2* __restrict__ edges,
-			const uint32_t* __restrict__ faces, u26_prp_hit* __restrict__ out)
+			const uint32_t* __restrict__ seg, const uint32_t* __restrict__ pos, const uint32_t* __restrict__ sel_begin,
+			const float* __restrict__ pay, HitKeyCodec cd, const uint2* __restrict__ edges, const uint32_t* __restrict__ faces,
+			u26_prp_hit* __restrict__ out)
 		{
-			__shared__ uint32_t wsum[8];
-			__shared__ uint32_t base;
-			const uint32_t t = list[blockIdx.x];
+			const uint32_t q = blockIdx.x / kCaptureBlocks;
+			const uint32_t t = list[q];
 			const uint32_t b = best[t];
-			const uint32_t lo = seg[t], hi = seg[t + 1];
-			if (threadIdx.x == 0)
-				base = out_off[blockIdx.x];
-			__syncthreads();
-			const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-			for (uint32_t i0 = lo; i0 < hi; i0 += blockDim.x)
+			const uint32_t lo = seg[t], hi = seg[t + 1], p0 = sel_begin[t], o0 = out_off[q];
+			for (uint64_t i = uint64_t(lo) + (blockIdx.x % kCaptureBlocks) * 256u + threadIdx.x; i < hi; i += kCaptureBlocks * 256u)
 			{
-				const uint32_t i = i0 + threadIdx.x;
-				const bool sel = i < hi && root[i] == b;
-				const uint32_t m = __ballot_sync(0xFFFFFFFFu, sel);
-				if (lane == 0)
-					wsum[warp] = __popc(m);
-				__syncthreads();
-				uint32_t off = base;
-				for (int w = 0; w < warp; w++)
-					off += wsum[w];
-				off += __popc(m & ((1u << lane) - 1u));
-				if (sel)
+				if (root[i] != b)
+					continue;
+				const uint64_t k = keys[i];
+				u26_prp_hit h;
+				h.type = cd.type(k);
+				h.src_id = cd.src(k);
+				h.dst_id = cd.dst(k);
+				uint32_t sv3[3], dv3[3];
+				hit_verts(h.type, h.src_id, h.dst_id, edges, faces, sv3, dv3);
+				for (int c = 0; c < 3; c++)
 				{
-					const uint64_t k = keys[i];
-					u26_prp_hit h;
-					h.type = cd.type(k);
-					h.src_id = cd.src(k);
-					h.dst_id = cd.dst(k);
-					uint32_t sv3[3], dv3[3];
-					hit_verts(h.type, h.src_id, h.dst_id, edges, faces, sv3, dv3);
-					for (int q = 0; q < 3; q++)
-					{
-						h.src_verts[q] = sv3[q];
-						h.dst_verts[q] = dv3[q];
-					}
-					h.bary[0] = pay[3 * i];
-					h.bary[1] = pay[3 * i + 1];
-					h.dist = pay[3 * i + 2];
-					out[off] = h;
+					h.src_verts[c] = sv3[c];
+					h.dst_verts[c] = dv3[c];
 				}
-				__syncthreads();
-				if (threadIdx.x == 0)
-				{
-					uint32_t tot = 0;
-					for (int w = 0; w < 8; w++)
-						tot += wsum[w];
-					base += tot;
-				}
-				__syncthreads();
+				h.bary[0] = pay[3 * i];
+				h.bary[1] = pay[3 * i + 1];
+				h.dist = pay[3 * i + 2];
+				out[o0 + (pos[i] - p0)] = h;
 			}
 		}
 
-		// selected-hit offset of each task: the scanned position of its first hit
+		// selected-hit offset of each task: the scanned position of its first hit (a warp per task; one thread
+		// counting up to 1,023 flags took 0.11 ms a level)
 		__global__ void sel_begin_kernel(uint32_t ntasks, const uint32_t* __restrict__ seg, const uint32_t* __restrict__ bsum_scanned,
 			const uint64_t* __restrict__ keys, const uint32_t* __restrict__ root, const uint32_t* __restrict__ best, HitKeyCodec cd,
 			uint32_t n, uint32_t* __restrict__ sel_begin)
 		{
-			const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+			const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+			const uint32_t lane = threadIdx.x & 31u;
 			if (t >= ntasks)
 				return;
 			// count selected flags in [block start, seg[t]) on top of the block prefix
 			const uint32_t i0 = seg[t];
 			const uint32_t blk = i0 / 1024u;
-			uint32_t p = bsum_scanned[blk];
-			for (uint32_t i = blk * 1024u; i < i0; i++)
+			uint32_t p = 0;
+			for (uint32_t i = blk * 1024u + lane; i < i0; i += 32u)
 				p += selected_flag(keys, root, best, cd, i, n);
-			sel_begin[t] = p;
+			p = __reduce_add_sync(0xFFFFFFFFu, p);
+			if (lane == 0)
+				sel_begin[t] = bsum_scanned[blk] + p;
 		}
 
 		// ---- FP64 evaluation of the selected supports (prp_eval_penetration_v2's terms,
@@ -4421,10 +4485,21 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 		U26_CUDA(ctx, S->d_cur_opp.reserve(sizeof(float) * size_t(nslots) * vs));
 		U26_CUDA(ctx, cudaMemsetAsync(S->d_cur_own.ptr, 0xFF, sizeof(float) * size_t(nslots) * vs, st));
 		U26_CUDA(ctx, cudaMemsetAsync(S->d_cur_opp.ptr, 0xFF, sizeof(float) * size_t(nslots) * vs, st));
-		distances_kernel<<<nslots, 256, 0, st>>>(S->d_slots.as<Slot>(), S->d_slot_ids.as<uint32_t>(), S->d_bnd.as<uint32_t>(),
-			S->d_vav_off.as<uint32_t>(), S->d_vav.as<uint32_t>(), S->d_rest_x.as<float>(), vs, S->d_hop.as<uint32_t>(),
-			S->d_geo.as<float>(), S->d_order.as<uint32_t>(), S->d_level_end.as<uint32_t>(), S->d_work.as<uint32_t>(),
-			S->d_mark.as<uint32_t>(), ctx->dev_err);
+		auto distances = [&](auto* kernel, size_t smem)
+		{
+			kernel<<<2u * nslots, kDistThreads, smem, st>>>(S->d_slots.as<Slot>(), S->d_slot_ids.as<uint32_t>(), S->d_bnd.as<uint32_t>(),
+				S->d_vav_off.as<uint32_t>(), S->d_vav.as<uint32_t>(), S->d_rest_x.as<float>(), vs, S->d_hop.as<uint32_t>(),
+				S->d_geo.as<float>(), S->d_order.as<uint32_t>(), S->d_level_end.as<uint32_t>(), S->d_work.as<uint32_t>(),
+				S->d_mark.as<uint32_t>(), ctx->dev_err);
+		};
+		// vs: the largest object's vertices
+		if (vs <= kSharedVerts)
+		{
+			U26_CUDA(ctx, cudaFuncSetAttribute(distances_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dist_smem(kSharedVerts))));
+			distances(&distances_kernel<true>, dist_smem(vs));
+		}
+		else
+			distances(&distances_kernel<false>, 0);
 		U26_TRY(after_launch(ctx, "distances_kernel"));
 		contour_directions();
 		mark("directions (beside the distances)");
@@ -4643,7 +4718,7 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 				P->ccr_use_rest, P->ccr_blend, P->ccr_tau, kBlocksPerSlot, S->d_cur_own.as<float>(), S->d_cur_opp.as<float>());
 			U26_TRY(after_launch(ctx, "ccr_current_kernel"));
 		}
-		candidates_kernel<<<uint32_t(sids.size()), 256, 0, st>>>(S->d_slots.as<Slot>(), S->d_slot_ids.as<uint32_t>(), S->d_bnd.as<uint32_t>(),
+		candidates_kernel<<<uint32_t(sids.size()), kCandThreads, 0, st>>>(S->d_slots.as<Slot>(), S->d_slot_ids.as<uint32_t>(), S->d_bnd.as<uint32_t>(),
 			d_x, S->d_edges.as<uint2>(), S->d_faces.as<uint32_t>(), S->d_vae_off.as<uint32_t>(), S->d_vae.as<uint32_t>(),
 			S->d_vaf_off.as<uint32_t>(), S->d_vaf.as<uint32_t>(), vs, es_, fs, S->d_hop.as<uint32_t>(), S->d_geo.as<float>(),
 			S->d_order.as<uint32_t>(), S->d_level_end.as<uint32_t>(), P->ccr_use_rest, P->ccr_use_current, P->ccr_blend, P->ccr_tau,
@@ -4995,7 +5070,7 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 				S->d_fn.as<float>(), S->d_slots.as<Slot>(), S->d_hop.as<uint32_t>(), vs, S->d_pos.as<uint32_t>(), S->d_terms.as<float>(),
 				S->d_task_max.as<uint32_t>(), hits_out ? S->d_sel.as<u26_prp_hit>() : nullptr);
 			U26_TRY(after_launch(ctx, "sel_terms_kernel"));
-			sel_begin_kernel<<<div_up(nt, 256), 256, 0, st>>>(nt, S->d_seg.as<uint32_t>(), S->d_bsum.as<uint32_t>(), S->d_keys.as<uint64_t>(),
+			sel_begin_kernel<<<div_up(nt, 8), 256, 0, st>>>(nt, S->d_seg.as<uint32_t>(), S->d_bsum.as<uint32_t>(), S->d_keys.as<uint64_t>(),
 				S->d_root.as<uint32_t>(), d_best, cd, nh, S->d_selbegin.as<uint32_t>());
 			U26_TRY(after_launch(ctx, "sel_begin_kernel"));
 		}
@@ -5189,9 +5264,10 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 						std::swap(grown.bytes, S->d_store.bytes);
 						grown.release(); // after the copy: cudaFree waits for the device
 					}
-					capture_kernel<<<uint32_t(list.size()), 256, 0, st>>>(S->d_cap_list.as<uint32_t>(), S->d_cap_off.as<uint32_t>(),
-						S->d_keys.as<uint64_t>(), S->d_root.as<uint32_t>(), S->d_best.as<uint32_t>(), S->d_seg.as<uint32_t>(), S->d_pay.as<float>(),
-						HitKeyCodec{ b }, S->d_edges.as<uint2>(), S->d_faces.as<uint32_t>(), S->d_store.as<u26_prp_hit>() + S->store_used);
+					capture_kernel<<<uint32_t(list.size()) * kCaptureBlocks, 256, 0, st>>>(S->d_cap_list.as<uint32_t>(),
+						S->d_cap_off.as<uint32_t>(), S->d_keys.as<uint64_t>(), S->d_root.as<uint32_t>(), S->d_best.as<uint32_t>(),
+						S->d_seg.as<uint32_t>(), S->d_pos.as<uint32_t>(), S->d_selbegin.as<uint32_t>(), S->d_pay.as<float>(), HitKeyCodec{ b },
+						S->d_edges.as<uint2>(), S->d_faces.as<uint32_t>(), S->d_store.as<u26_prp_hit>() + S->store_used);
 					U26_TRY(after_launch(ctx, "capture_kernel"));
 					for (size_t q = 0; q < list.size(); q++)
 						R[tasks[list[q]].contour_local].res[tasks[list[q]].combo].store_off = S->store_used + off[q];
