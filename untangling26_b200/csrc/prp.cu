@@ -1899,13 +1899,16 @@ namespace u26
 		}
 
 		// ---- run directory: every (task, type, source) run of the sorted hits, in an
-		// open-addressing hash table keyed by that prefix (value: run id; run r spans
-		// [heads[r], heads[r + 1]))
+		// open-addressing hash table keyed by that prefix. A slot holds the key and the run [begin, end), so a
+		// lookup is one 16-byte load (a key, a run id and two list entries were three dependent ones).
+		struct __align__(16) RunSlot
+		{
+			unsigned long long key; // prefix + 1 (0: empty slot)
+			uint32_t begin, end;
+		};
 		struct RunDir
 		{
-			const uint64_t* hkeys; // prefix + 1 (0: empty slot)
-			const uint32_t* hvals;
-			const uint32_t* heads;
+			const RunSlot* slots;
 			uint32_t mask;
 		};
 		__device__ __forceinline__ uint32_t run_hash(uint64_t p)
@@ -1917,37 +1920,47 @@ namespace u26
 			p ^= p >> 33;
 			return uint32_t(p);
 		}
-		__global__ void run_flags_kernel(const uint64_t* __restrict__ keys, uint32_t n, int b, uint32_t* __restrict__ flag)
+		__device__ __forceinline__ bool run_head(const uint64_t* __restrict__ keys, uint32_t i, int b)
 		{
-			const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-			if (i > n)
-				return;
-			flag[i] = (i < n && (i == 0 || (keys[i] >> b) != (keys[i - 1] >> b))) ? 1u : 0u;
+			return i == 0 || (keys[i] >> b) != (keys[i - 1] >> b);
 		}
-		// flag[] scanned in place: flag[i] = run id of a head i; flag[n] = number of runs
-		__global__ void run_insert_kernel(const uint64_t* __restrict__ keys, uint32_t n, int b, const uint32_t* __restrict__ scanned,
-			uint32_t* __restrict__ heads, uint64_t* __restrict__ hkeys, uint32_t* __restrict__ hvals, uint32_t mask, uint32_t* __restrict__ dev_err)
+		__global__ void __launch_bounds__(256) run_count_kernel(const uint64_t* __restrict__ keys, uint32_t n, int b, uint32_t* __restrict__ count)
 		{
 			const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-			if (i > n)
+			const int c = __syncthreads_count(i < n && run_head(keys, i, b));
+			if (threadIdx.x == 0 && c)
+				atomicAdd(count, uint32_t(c));
+		}
+		__global__ void run_insert_kernel(const uint64_t* __restrict__ keys, uint32_t n, int b, RunSlot* __restrict__ slots, uint32_t mask,
+			uint32_t* __restrict__ dev_err)
+		{
+			const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+			if (i >= n || !run_head(keys, i, b))
 				return;
-			if (i == n)
+			// the run's end: doubling steps inside the run, then a binary search
+			const uint64_t prefix = keys[i] >> b;
+			uint32_t in = i, step = 1;
+			while (n - in > step && (keys[in + step] >> b) == prefix)
 			{
-				heads[scanned[n]] = n;
-				return;
+				in += step;
+				step <<= 1;
 			}
-			if (!(i == 0 || (keys[i] >> b) != (keys[i - 1] >> b)))
-				return;
-			const uint32_t r = scanned[i];
-			heads[r] = i;
-			const uint64_t k = (keys[i] >> b) + 1u;
+			uint32_t lo = in + 1u, hi = in + min(step, n - in);
+			while (lo < hi)
+			{
+				const uint32_t mid = (lo + hi) >> 1;
+				if ((keys[mid] >> b) == prefix)
+					lo = mid + 1u;
+				else
+					hi = mid;
+			}
+			const unsigned long long k = prefix + 1u;
 			uint32_t h = run_hash(k) & mask;
 			for (uint32_t it = 0; it <= mask; it++)
 			{
-				const unsigned long long old = atomicCAS(reinterpret_cast<unsigned long long*>(hkeys + h), 0ull, (unsigned long long)k);
-				if (old == 0ull)
+				if (atomicCAS(&slots[h].key, 0ull, k) == 0ull)
 				{
-					hvals[h] = r;
+					*reinterpret_cast<uint2*>(&slots[h].begin) = make_uint2(i, lo);
 					return;
 				}
 				h = (h + 1u) & mask;
@@ -1962,19 +1975,21 @@ namespace u26
 			rb = re = 0;
 			for (uint32_t it = 0; it <= d.mask; it++)
 			{
-				const uint64_t v = d.hkeys[h];
-				if (v == k)
+				const uint4 v = __ldg(reinterpret_cast<const uint4*>(d.slots + h));
+				const uint64_t key = (uint64_t(v.y) << 32) | v.x;
+				if (key == k)
 				{
-					const uint32_t r = d.hvals[h];
-					rb = d.heads[r];
-					re = d.heads[r + 1];
+					rb = v.z;
+					re = v.w;
 					return;
 				}
-				if (v == 0ull)
+				if (key == 0ull)
 					return;
 				h = (h + 1u) & d.mask;
 			}
 		}
+
+		constexpr uint32_t kFewHits = 1u << 18; // their table (8 MB) is cleared in the time of a launch
 
 		// find_adjacent_hits rules as exact key lookups inside the task segment. Lookups that
 		// share a (type, source) first find that source's run of hits once, then search the
@@ -2777,13 +2792,13 @@ namespace u26
 			}
 			nchunk[t] = c;
 		}
-		__global__ void chunk_sum_kernel(uint32_t ntasks, uint32_t nchunks, const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ best,
+		__global__ void chunk_sum_kernel(uint32_t ntasks, const uint32_t* __restrict__ chunk_off, const uint32_t* __restrict__ best,
 			const uint32_t* __restrict__ comp_size, const uint32_t* __restrict__ sel_begin, const float* __restrict__ terms,
 			float* __restrict__ csum)
 		{
 			const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 			const int lane = threadIdx.x & 31;
-			if (g >= nchunks)
+			if (g >= chunk_off[ntasks])
 				return;
 			uint32_t lo = 0, hi = ntasks;
 			while (hi - lo > 1)
@@ -3445,7 +3460,7 @@ struct u26_scene
 	DevBuf d_store;	 // the pass's captured supports (u26_prp_hit), grown with its contents kept
 	uint64_t store_used = 0;
 	DevBuf d_fetch_off, d_fetch_cnt, d_fetch_pos;
-	DevBuf d_vrank, d_erank, d_cand_off, d_ckeys, d_cvals, d_cap_list, d_cap_off, d_capture, d_chunk_off, d_csum, scan_tmp, d_vsolid, d_fvk, d_fvv, d_rflag, d_heads, d_hkeys, d_hvals, d_zero_th;
+	DevBuf d_vrank, d_erank, d_cand_off, d_ckeys, d_cvals, d_cap_list, d_cap_off, d_capture, d_chunk_off, d_csum, scan_tmp, d_vsolid, d_fvk, d_fvv, d_runs, d_hslots, d_zero_th;
 	RadixSorter sorter, esorter, csorter, fvsorter;
 	std::vector<uint8_t> vsolid; // per vertex: its object is rigid / tetrahedral
 	bool any_solid = false;
@@ -3684,7 +3699,7 @@ U26_API void u26_scene_destroy(u26_scene* s)
 		&s->d_step_hits, &s->d_step_out, &s->d_f64in, &s->d_f64hits, &s->d_f64delta, &s->d_f64out, &s->d_queue, &s->d_fgrow, &s->d_egrow, &s->d_front, &s->d_cur_own,
 		&s->d_cur_opp, &s->d_tab, &s->d_cov, &s->d_vrank, &s->d_erank, &s->d_cand_off, &s->d_ckeys, &s->d_cvals,
 		&s->d_cap_list, &s->d_cap_off, &s->d_capture, &s->d_chunk_off, &s->d_csum, &s->scan_tmp, &s->d_vsolid,
-		&s->d_fvk, &s->d_fvv, &s->d_rflag, &s->d_heads, &s->d_hkeys, &s->d_hvals,
+		&s->d_fvk, &s->d_fvv, &s->d_runs, &s->d_hslots,
 		&s->d_zero_th, &s->d_trange, &s->d_store, &s->d_fetch_off, &s->d_fetch_cnt, &s->d_fetch_pos };
 	for (DevBuf* b : bufs)
 		b->release();
@@ -4917,24 +4932,28 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 				S->d_csize.as<uint32_t>(), S->d_catt.as<uint32_t>());
 			U26_TRY(after_launch(ctx, "init_hits_kernel"));
 			// run directory of this level's hits
-			U26_CUDA(ctx, S->d_rflag.reserve(sizeof(uint32_t) * (size_t(nh) + 1)));
-			run_flags_kernel<<<div_up(nh + 1, 256), 256, 0, st>>>(S->d_keys.as<uint64_t>(), nh, b, S->d_rflag.as<uint32_t>());
-			U26_TRY(after_launch(ctx, "run_flags_kernel"));
-			U26_TRY(device_exclusive_scan(ctx, S->d_rflag.as<uint32_t>(), nh + 1, S->scan_tmp));
-			U26_CUDA(ctx, cudaMemcpyAsync(ctx->host_word, S->d_rflag.as<uint32_t>() + nh, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-			U26_CUDA(ctx, cudaStreamSynchronize(st));
-			const uint32_t nruns = *ctx->host_word;
-			uint32_t hsize = 1024;
-			while (hsize < 2 * nruns)
+			// two slots per run; levels of few hits take their number for the runs', and save the count's
+			// host read
+			uint32_t nruns = nh;
+			if (nh > kFewHits)
+			{
+				U26_CUDA(ctx, S->d_runs.reserve(sizeof(uint32_t)));
+				U26_CUDA(ctx, cudaMemsetAsync(S->d_runs.ptr, 0, sizeof(uint32_t), st));
+				run_count_kernel<<<div_up(nh, 256), 256, 0, st>>>(S->d_keys.as<uint64_t>(), nh, b, S->d_runs.as<uint32_t>());
+				U26_TRY(after_launch(ctx, "run_count_kernel"));
+				U26_CUDA(ctx, cudaMemcpyAsync(ctx->host_word, S->d_runs.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+				U26_CUDA(ctx, cudaStreamSynchronize(st));
+				nruns = *ctx->host_word;
+			}
+			uint64_t hsize = 1024;
+			while (hsize < 2 * uint64_t(nruns))
 				hsize <<= 1;
-			U26_CUDA(ctx, S->d_heads.reserve(sizeof(uint32_t) * (size_t(nruns) + 1)));
-			U26_CUDA(ctx, S->d_hkeys.reserve(sizeof(uint64_t) * hsize));
-			U26_CUDA(ctx, S->d_hvals.reserve(sizeof(uint32_t) * hsize));
-			U26_CUDA(ctx, cudaMemsetAsync(S->d_hkeys.ptr, 0, sizeof(uint64_t) * hsize, st));
-			run_insert_kernel<<<div_up(nh + 1, 256), 256, 0, st>>>(S->d_keys.as<uint64_t>(), nh, b, S->d_rflag.as<uint32_t>(),
-				S->d_heads.as<uint32_t>(), S->d_hkeys.as<uint64_t>(), S->d_hvals.as<uint32_t>(), hsize - 1, ctx->dev_err);
+			U26_CUDA(ctx, S->d_hslots.reserve(sizeof(RunSlot) * hsize));
+			U26_CUDA(ctx, cudaMemsetAsync(S->d_hslots.ptr, 0, sizeof(RunSlot) * hsize, st));
+			run_insert_kernel<<<div_up(nh, 256), 256, 0, st>>>(S->d_keys.as<uint64_t>(), nh, b, S->d_hslots.as<RunSlot>(), uint32_t(hsize - 1),
+				ctx->dev_err);
 			U26_TRY(after_launch(ctx, "run_insert_kernel"));
-			const RunDir rdir{ S->d_hkeys.as<uint64_t>(), S->d_hvals.as<uint32_t>(), S->d_heads.as<uint32_t>(), hsize - 1 };
+			const RunDir rdir{ S->d_hslots.as<RunSlot>(), uint32_t(hsize - 1) };
 			union_kernel<<<div_up(nh, 128), 128, 0, st>>>(S->d_keys.as<uint64_t>(), nh, cd, S->d_seg.as<uint32_t>(), S->d_edges.as<uint2>(),
 				S->d_faces.as<uint32_t>(), S->d_fae.as<uint32_t>(), S->d_vav_off.as<uint32_t>(), S->d_vav.as<uint32_t>(),
 				S->d_vae_off.as<uint32_t>(), S->d_vae.as<uint32_t>(), S->d_vaf_off.as<uint32_t>(), S->d_vaf.as<uint32_t>(),
@@ -5057,11 +5076,16 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 			U26_TRY(after_launch(ctx, "sel_block_sums_kernel"));
 			scan_one_block_kernel<<<1, 1024, 0, st>>>(S->d_bsum.as<uint32_t>(), nblk, S->d_bsum.as<uint32_t>() + nblk + 1);
 			U26_TRY(after_launch(ctx, "scan_one_block_kernel"));
-			U26_CUDA(ctx, cudaMemcpyAsync(ctx->host_word, S->d_bsum.as<uint32_t>() + nblk + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-			U26_CUDA(ctx, cudaStreamSynchronize(st));
-			nsel = *ctx->host_word;
+			// (the number of selected hits is read back only where the hits are: the terms' buffer holds
+			// every hit's)
+			if (hits_out || trace)
+			{
+				U26_CUDA(ctx, cudaMemcpyAsync(ctx->host_word, S->d_bsum.as<uint32_t>() + nblk + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+				U26_CUDA(ctx, cudaStreamSynchronize(st));
+				nsel = *ctx->host_word;
+			}
 			U26_CUDA(ctx, S->d_pos.reserve(sizeof(uint32_t) * nh1));
-			U26_CUDA(ctx, S->d_terms.reserve(sizeof(float) * 3 * size_t(std::max(nsel, 1u))));
+			U26_CUDA(ctx, S->d_terms.reserve(sizeof(float) * 3 * size_t(nh1)));
 			if (hits_out)
 				U26_CUDA(ctx, S->d_sel.reserve(sizeof(u26_prp_hit) * size_t(std::max(nsel, 1u))));
 			sel_terms_kernel<<<nblk, 256, 0, st>>>(S->d_keys.as<uint64_t>(), S->d_root.as<uint32_t>(), d_best, cd, nh, S->d_bsum.as<uint32_t>(),
@@ -5077,18 +5101,18 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 		else
 			U26_CUDA(ctx, cudaMemsetAsync(S->d_selbegin.ptr, 0, sizeof(uint32_t) * (nt + 1), st));
 		U26_CUDA(ctx, S->d_out.reserve(sizeof(TaskOut) * nt));
-		// chunk sums of the supports longer than kSumChunk
+		// chunk sums of the supports longer than kSumChunk (their number stays on the device; each has more than
+		// half a chunk on average)
 		U26_CUDA(ctx, S->d_chunk_off.reserve(sizeof(uint32_t) * (nt + 1)));
-		chunk_count_kernel<<<div_up(nt + 1, 256), 256, 0, st>>>(nt, d_best, S->d_csize.as<uint32_t>(), S->d_chunk_off.as<uint32_t>());
-		U26_TRY(after_launch(ctx, "chunk_count_kernel"));
-		U26_TRY(device_exclusive_scan(ctx, S->d_chunk_off.as<uint32_t>(), nt + 1, S->scan_tmp));
-		U26_CUDA(ctx, cudaMemcpyAsync(ctx->host_word, S->d_chunk_off.as<uint32_t>() + nt, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-		U26_CUDA(ctx, cudaStreamSynchronize(st));
-		const uint32_t nchunks = *ctx->host_word;
-		U26_CUDA(ctx, S->d_csum.reserve(sizeof(float) * 3 * size_t(std::max(nchunks, 1u))));
-		if (nchunks)
+		U26_CUDA(ctx, S->d_csum.reserve(sizeof(float) * 3));
+		if (max_seg > kSumChunk)
 		{
-			chunk_sum_kernel<<<div_up(32 * nchunks, 256), 256, 0, st>>>(nt, nchunks, S->d_chunk_off.as<uint32_t>(), d_best,
+			const uint32_t most = 2u * (nh / kSumChunk) + 1u;
+			chunk_count_kernel<<<div_up(nt + 1, 256), 256, 0, st>>>(nt, d_best, S->d_csize.as<uint32_t>(), S->d_chunk_off.as<uint32_t>());
+			U26_TRY(after_launch(ctx, "chunk_count_kernel"));
+			U26_TRY(device_exclusive_scan(ctx, S->d_chunk_off.as<uint32_t>(), nt + 1, S->scan_tmp));
+			U26_CUDA(ctx, S->d_csum.reserve(sizeof(float) * 3 * size_t(most)));
+			chunk_sum_kernel<<<uint32_t(div_up64(32 * uint64_t(most), 256)), 256, 0, st>>>(nt, S->d_chunk_off.as<uint32_t>(), d_best,
 				S->d_csize.as<uint32_t>(), S->d_selbegin.as<uint32_t>(), S->d_terms.as<float>(), S->d_csum.as<float>());
 			U26_TRY(after_launch(ctx, "chunk_sum_kernel"));
 		}
