@@ -786,7 +786,9 @@ namespace u26
 		// Conservative node margins, applied to every node once per pass so that the traversals
 		// read grown boxes: eps = 1e-5 (1 + max |bound|) per axis for the ray slab tests, one eps
 		// from all six bounds for the swept-edge box tests (the epsilon-grown node tests that
-		// keep the traversal a superset of the exact primitive tests).
+		// keep the traversal a superset of the exact primitive tests). Face trees (isotropic 0) hold minima and
+		// maxima; edge trees (isotropic 1) centres and half extents, which the swept-edge test takes: 27
+		// instructions a box instead of 55, ray casting of 16 two-body scenes 113 ms, 103 ms.
 		// The w lanes carry the node's links, so one 32-byte load serves a visit: inner node
 		// (mn.w, mx.w) = (left, right child); leaf (mn.w, mx.w) = (primitive, ~0).
 		// node_off / prim_off place one object's tree in the forest of all objects' trees
@@ -801,8 +803,22 @@ namespace u26
 			if (isotropic)
 			{
 				const float e = 1e-5f * (1.0f + fmaxf(fmaxf(fabsf(b.mn.x), fabsf(b.mx.x)), fmaxf(fmaxf(fabsf(b.mn.y), fabsf(b.mx.y)), fmaxf(fabsf(b.mn.z), fabsf(b.mx.z)))));
-				g.mn = make_float4(b.mn.x - e, b.mn.y - e, b.mn.z - e, 0.0f);
-				g.mx = make_float4(b.mx.x + e, b.mx.y + e, b.mx.z + e, 0.0f);
+				// centre and half extents, as the swept-edge box test takes them; an axis with an infinite or NaN
+				// bound covers everything (the exact tests decide)
+				auto axis = [&](float lo, float hi, float& c, float& h)
+				{
+					c = 0.5f * (lo + hi);
+					h = 0.5f * (hi - lo);
+					if (!isfinite(c) || !isfinite(h))
+					{
+						c = 0.0f;
+						h = 3e38f;
+					}
+				};
+				axis(b.mn.x - e, b.mx.x + e, g.mn.x, g.mx.x);
+				axis(b.mn.y - e, b.mx.y + e, g.mn.y, g.mx.y);
+				axis(b.mn.z - e, b.mx.z + e, g.mn.z, g.mx.z);
+				g.mn.w = g.mx.w = 0.0f;
 			}
 			else
 			{
@@ -964,8 +980,9 @@ namespace u26
 		// Bound by the latency of the divergent node loads (a third of the issue slots wait for them). 64.5 M
 		// requests of 16 two-body scenes (161 node and 28 leaf tests each): 225 ms with the warp walking the union
 		// of its requests' paths and testing a leaf with the lanes that met it (three times the nodes, 19 of 32
-		// lanes busy), 113 ms now; two 64 x 64 sheets 14.3 ms, 6.3 ms; folded 64 x 64 sheet, 26 directions, 19.0
-		// ms, 11.4 ms.
+		// lanes busy), 103 ms now; two 64 x 64 sheets 14.3 ms, 5.9 ms; folded 64 x 64 sheet, 26 directions, 19.0
+		// ms, 10.2 ms. Measured and dropped: records of four grandchildren (half the dependent steps; 121 ms where
+		// this took 113: the registers of four boxes in flight).
 		constexpr int kStack = 64;
 		struct RayWarp
 		{
@@ -1427,32 +1444,26 @@ namespace u26
 				W.u[5][lane] = plane ? 1u : 0u, W.u[6][lane] = ev.x, W.u[7][lane] = ev.y;
 				__syncwarp();
 				const uint32_t tested0 = tested;
+				const f3 sc = 0.5f * (smn + smx), sh = 0.5f * (smx - smn);
+				const float proj_c = 0.5f * (proj_lo + proj_hi), proj_h = 0.5f * (proj_hi - proj_lo);
+				const f3 wn = plane ? pn : mk3(0.0f); // (no plane: every box meets the slab)
+				const float wd = plane ? pd : 0.0f;
 				ray_walk(
 					W, egrow, estart, visited, tested, dev_err,
+					// g.mn, g.mx: centre and half extents. The box meets the swept box; its extent along dir meets the
+					// swept edge's (a box that misses it holds no edge the swept edge reaches); and it meets the
+					// slab |dot(pn, q) - pd| <= 1e-6 around the swept edge's plane (a box clear of it holds only
+					// edges the leaf's separating-plane test rejects; cached_bvh.cpp:433-473 prunes its nodes the same
+					// way). Explicit fmas: the boxes carry the 1e-5 (1 + |c|) margin, far above this
+					// test's rounding, so no edge the leaf test keeps is pruned.
 					[&](const NodeBox& g)
 					{
-						bool hit = (smn.x <= g.mx.x) & (smx.x >= g.mn.x) & (smn.y <= g.mx.y) & (smx.y >= g.mn.y) & (smn.z <= g.mx.z) &
-							(smx.z >= g.mn.z);
-						// the swept edge lies in the plane (pn, pd): a box that keeps clear of the slab
-						// |dot(pn, q) - pd| <= 1e-6 holds only edges the leaf's separating-plane test
-						// rejects (cached_bvh.cpp:433-473 prunes its nodes the same way). The boxes carry
-						// the 1e-5 (1 + |c|) margin, far above the rounding of this test, so no edge the
-						// leaf test keeps is pruned.
-						// and a box whose extent along dir misses the swept edge's holds no edge it reaches
-						if (hit)
-						{
-							const f3 c = mk3(0.5f * (g.mn.x + g.mx.x), 0.5f * (g.mn.y + g.mx.y), 0.5f * (g.mn.z + g.mx.z));
-							const f3 h = mk3(0.5f * (g.mx.x - g.mn.x), 0.5f * (g.mx.y - g.mn.y), 0.5f * (g.mx.z - g.mn.z));
-							const float cp = dot(c, dir);
-							const float pr = (h.x * fabsf(dir.x) + h.y * fabsf(dir.y)) + h.z * fabsf(dir.z);
-							hit = !(cp + pr < proj_lo || cp - pr > proj_hi);
-							if (hit && plane)
-							{
-								const float rad = (h.x * fabsf(pn.x) + h.y * fabsf(pn.y)) + h.z * fabsf(pn.z);
-								hit = fabsf(dot(pn, c) - pd) <= rad + 1e-6f;
-							}
-						}
-						return hit;
+						const float cp = __fmaf_rn(g.mn.z, dir.z, __fmaf_rn(g.mn.y, dir.y, g.mn.x * dir.x));
+						const float pr = __fmaf_rn(g.mx.z, fabsf(dir.z), __fmaf_rn(g.mx.y, fabsf(dir.y), g.mx.x * fabsf(dir.x)));
+						const float cn = __fmaf_rn(g.mn.z, wn.z, __fmaf_rn(g.mn.y, wn.y, g.mn.x * wn.x));
+						const float rn = __fmaf_rn(g.mx.z, fabsf(wn.z), __fmaf_rn(g.mx.y, fabsf(wn.y), g.mx.x * fabsf(wn.x)));
+						return (fabsf(g.mn.x - sc.x) <= g.mx.x + sh.x) & (fabsf(g.mn.y - sc.y) <= g.mx.y + sh.y) &
+							(fabsf(g.mn.z - sc.z) <= g.mx.z + sh.z) & (fabsf(cp - proj_c) <= pr + proj_h) & (fabsf(cn - wd) <= rn + 1e-6f);
 					},
 					[&](uint32_t e2, uint32_t from, uint32_t n) { told += test_edges<RECHECK>(L, e2, from, n); count_told(); });
 				etested += tested - tested0;
@@ -1508,8 +1519,8 @@ namespace u26
 			{ 8, 6, false }, { 16, 4, false }, { 16, 5, false }, { 16, 6, false }, { 4, 4, true }, { 4, 5, true }, { 4, 6, true }, { 8, 4, true },
 			{ 8, 5, true }, { 8, 6, true }, { 16, 4, true }, { 16, 5, true }, { 16, 6, true } };
 		// The default: the queue at 5 blocks per SM, in 8 parts. Parts share a ray's setup but not its balance: 16
-		// scenes of 2k-60k triangles take 113 ms in 4 parts, 121 in 8; a folded sheet with 26 directions 13.4, 11.4
-		// (10.5 in 16); two 64 x 64 sheets 6.3, 6.8. Launches of kManyRequests and more (the first kind) use 4.
+		// scenes of 2k-60k triangles take 102 ms in 4 parts, 111 in 8; a folded sheet with 26 directions 11.8, 10.1
+		// (9.4 in 16); two 64 x 64 sheets 5.6, 6.2. Launches of kManyRequests and more (the first kind) use 4.
 		constexpr int kNumRaycastConfigs = 18, kDefaultRaycastConfig = 13;
 		constexpr uint32_t kManyRequests = 1u << 20;
 		using RaycastFn = decltype(&raycast_kernel<false, 5, false>);
