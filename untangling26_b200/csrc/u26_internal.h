@@ -1,6 +1,7 @@
 // Host-side internals of libu26: the context object, grow-only device buffers and
 // error plumbing shared by the .cu translation units.
 #pragma once
+#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -29,7 +30,8 @@ namespace u26
 	// device and pinned-host allocations the library has made (u26_alloc_count)
 	extern std::atomic<uint64_t> g_alloc_count;
 
-	// Grow-only device allocation owned by a context-side object.
+	// Grow-only device allocation owned by a context-side object. A buffer that grows takes half as much again as
+	// it held: a scene's first pass asks for more at every level, and each growth waits for the device.
 	struct DevBuf
 	{
 		void* ptr = nullptr;
@@ -38,11 +40,21 @@ namespace u26
 		{
 			if (want <= bytes)
 				return cudaSuccess;
+			const size_t grown = std::max(want, bytes + bytes / 2);
 			if (ptr)
 				cudaFree(ptr);
 			ptr = nullptr;
 			bytes = 0;
-			cudaError_t e = cudaMalloc(&ptr, want);
+			cudaError_t e = cudaMalloc(&ptr, grown);
+			if (e != cudaSuccess && grown > want)
+			{
+				cudaGetLastError(); // of the larger request
+				e = cudaMalloc(&ptr, want);
+			}
+			else
+				want = grown;
+			if (e != cudaSuccess)
+				ptr = nullptr;
 			if (e == cudaSuccess)
 			{
 				bytes = want;
