@@ -328,7 +328,8 @@ typedef struct u26_prp_output_view
 									  * configuration (subtree parts, blocks per SM, grid form): (4,6) (4,7) (4,8) (8,6)
 									  * (8,7) (8,8) (16,6) (16,7) (16,8) with a warp per work item, then the same nine
 									  * with a persistent grid whose warps take work items from a queue */
-	uint32_t raycast_parts;			 /* configuration the scene's ray casts use from now on: subtree parts per request */
+	uint32_t raycast_parts;			 /* configuration the scene's ray casts use from now on: subtree parts per request (the
+									   * default's 8 are 4 in launches of 2^20 requests and more) */
 	uint32_t raycast_blocks_per_sm;	 /* ... resident 128-thread blocks per SM */
 	uint32_t tuned;					 /* 1 when this pass ran the autotuner (its choice holds for the scene's later passes) */
 	uint32_t raycast_queue;			 /* ... and 1 for the persistent work-queue grid */

@@ -781,12 +781,17 @@ namespace u26
 			SBox* s_leaf = reinterpret_cast<SBox*>(s_raw);
 			SBox* s_inner = s_leaf + kTreelet;
 			__shared__ uint32_t s_hmax;
-			if (blockIdx.x >= info[2])
-				return;
-			const uint32_t base = chunk_lo[blockIdx.x];
-			const uint32_t cnt = chunk_lo[blockIdx.x + 1] - base;
-			const uint32_t ni = n - 1;
 			const uint32_t t = threadIdx.x;
+			if (t == 0)
+				s_hmax = 0u;
+			__syncthreads();
+			// (the chunk's bounds are read beside the number of chunks, not after it: the list has an entry for
+			// every block)
+			const uint32_t nchunks = __ldg(info + 2), base = __ldg(chunk_lo + blockIdx.x), next = __ldg(chunk_lo + blockIdx.x + 1);
+			if (blockIdx.x >= nchunks)
+				return;
+			const uint32_t cnt = next - base;
+			const uint32_t ni = n - 1;
 			if (cnt > kTreelet || base + cnt > n)
 			{
 				// a plan that does not match the tree: nothing is read or written
@@ -794,8 +799,6 @@ namespace u26
 					atomicExch(health, 0u);
 				return;
 			}
-			if (t == 0)
-				s_hmax = 0u;
 			// inner nodes base + t and base + t + 512 (0: not all of their leaves are in the chunk)
 			uint32_t w[2] = { 0u, 0u };
 #pragma unroll
@@ -828,7 +831,6 @@ namespace u26
 					s_leaf[tq] = sbox(mn, mx);
 				}
 			}
-			__syncthreads();
 			const uint32_t wmax = __reduce_max_sync(0xFFFFFFFFu, max(w[0], w[1])) >> 22;
 			if ((t & 31) == 0 && wmax)
 				atomicMax(&s_hmax, wmax);
@@ -883,24 +885,32 @@ namespace u26
 		constexpr size_t kTopSmem = (sizeof(SBox) + sizeof(uint2)) * kTopShared;
 		__global__ void __launch_bounds__(1024) refit_top_kernel(NodeBox* __restrict__ boxes, const uint32_t* __restrict__ top_nodes,
 			const uint2* __restrict__ top_links, const uint32_t* __restrict__ level_end, const uint32_t* __restrict__ info,
-			const SBox* __restrict__ root_box, uint32_t* __restrict__ health)
+			const SBox* __restrict__ root_box, uint32_t room, uint32_t* __restrict__ health)
 		{
-			extern __shared__ __align__(16) unsigned char s_raw[];
+			extern __shared__ __align__(16) unsigned char s_raw[]; // boxes and links of `room` top nodes
 			SBox* s_box = reinterpret_cast<SBox*>(s_raw);
-			uint2* s_link = reinterpret_cast<uint2*>(s_box + kTopShared);
+			uint2* s_link = reinterpret_cast<uint2*>(s_box + room);
 			__shared__ uint32_t s_end[kMaxHeight + 1];
 			const uint32_t t = threadIdx.x;
-			const uint32_t m = info[0], nt = info[1];
-			const bool shared = m <= kTopShared;
-			auto valid = [&](uint32_t id, uint32_t j) { return (id & kTopRoot) ? (id & ~kTopRoot) < nt : id < j; };
+			// the first 1,024 nodes' data are read beside the counts, not after them (the arrays hold `room` nodes)
+			const bool in = t < room;
+			const uint2 link0 = in ? top_links[t] : make_uint2(0u, 0u);
+			const uint32_t node0 = in ? top_nodes[t] : 0u;
+			SBox first0 = SBox{}, second0 = SBox{};
+			if (in)
+			{
+				first0 = root_box[2u * t];
+				second0 = root_box[2u * t + 1u];
+			}
 			if (t <= kMaxHeight)
-				s_end[t] = min(level_end[t], m);
+				s_end[t] = level_end[t];
+			const uint32_t m = info[0], nt = info[1];
+			const bool shared = m <= room;
+			auto valid = [&](uint32_t id, uint32_t j) { return (id & kTopRoot) ? (id & ~kTopRoot) < nt : id < j; };
 			if (shared)
 			{
-#pragma unroll 4
-				for (uint32_t j = t; j < m; j += 1024u)
+				auto place = [&](uint32_t j, uint2 l, const SBox& first, const SBox& second)
 				{
-					uint2 l = top_links[j];
 					if (!valid(l.x, j) || !valid(l.y, j))
 					{
 						// a plan that does not match the tree
@@ -910,16 +920,21 @@ namespace u26
 					s_link[j] = l;
 					const bool rx = (l.x & kTopRoot) != 0u, ry = (l.y & kTopRoot) != 0u;
 					if (rx && ry)
-						s_box[j] = unite_s(root_box[2u * j], root_box[2u * j + 1u]);
+						s_box[j] = unite_s(first, second);
 					else if (rx || ry)
-						s_box[j] = root_box[2u * j + (rx ? 0u : 1u)];
-				}
+						s_box[j] = rx ? first : second;
+				};
+				if (t < m)
+					place(t, link0, first0, second0);
+#pragma unroll 4
+				for (uint32_t j = t + 1024u; j < m; j += 1024u)
+					place(j, top_links[j], root_box[2u * j], root_box[2u * j + 1u]);
 			}
 			__syncthreads();
 			uint32_t begin = 0;
 			for (uint32_t h = 1; h <= kMaxHeight && begin < m; h++)
 			{
-				const uint32_t end = s_end[h];
+				const uint32_t end = min(s_end[h], m);
 				for (uint32_t j = begin + t; j < end; j += 1024u)
 				{
 					SBox u;
@@ -960,8 +975,10 @@ namespace u26
 			}
 			if (shared)
 			{
+				if (t < m)
+					store_sbox(boxes + node0, s_box[t]);
 #pragma unroll 4
-				for (uint32_t j = t; j < m; j += 1024u)
+				for (uint32_t j = t + 1024u; j < m; j += 1024u)
 					store_sbox(boxes + top_nodes[j], s_box[j]);
 			}
 		}
@@ -1155,12 +1172,10 @@ U26_API u26_status u26_lbvh_reduce_aabb(u26_lbvh* t, const float* x, uint32_t nu
 	return U26_OK;
 }
 
-// The kernels' dynamic shared memory (above the 48 KB default), set once per device.
+// The kernels' dynamic shared memory (above the 48 KB default), set once per context.
 static u26_status size_plan_kernels(u26_ctx* ctx)
 {
-	static std::atomic<bool> sized[64];
-	const bool known = ctx->device >= 0 && ctx->device < 64;
-	if (known && sized[ctx->device].load(std::memory_order_acquire))
+	if (ctx->sized_plan.load(std::memory_order_acquire))
 		return U26_OK;
 	const void* chunk_kernels[] = { (const void*)refit_chunk_kernel<U26_TREE_VERT, false>, (const void*)refit_chunk_kernel<U26_TREE_VERT, true>,
 		(const void*)refit_chunk_kernel<U26_TREE_EDGE, false>, (const void*)refit_chunk_kernel<U26_TREE_EDGE, true>,
@@ -1170,8 +1185,7 @@ static u26_status size_plan_kernels(u26_ctx* ctx)
 	U26_CUDA(ctx, cudaFuncSetAttribute(refit_top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTopSmem)));
 	U26_CUDA(ctx, cudaFuncSetAttribute(plan_chunks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(uint32_t) * 4u * kChainShared)));
 	U26_CUDA(ctx, cudaFuncSetAttribute(plan_top_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(TopScratch) * kTopScratchShared)));
-	if (known)
-		sized[ctx->device].store(true, std::memory_order_release);
+	ctx->sized_plan.store(true, std::memory_order_release);
 	return U26_OK;
 }
 
@@ -1314,8 +1328,9 @@ static u26_status refit_impl(u26_lbvh* t, bool fused, const float* thickness, co
 	U26_TRY(after_launch(ctx, "refit_chunk_kernel"));
 	if (t->n <= kTreelet)
 		return U26_OK;
-	refit_top_kernel<<<1, 1024, kTopSmem, ctx->stream>>>(t->node_aabb.as<NodeBox>(), t->top_nodes.as<uint32_t>(), t->top_links.as<uint2>(),
-		t->level_end.as<uint32_t>(), info, t->root_box.as<SBox>(), t->health.as<uint32_t>());
+	const uint32_t room = std::min(kTopShared, plan_capacity(t->n));
+	refit_top_kernel<<<1, 1024, (sizeof(SBox) + sizeof(uint2)) * room, ctx->stream>>>(t->node_aabb.as<NodeBox>(), t->top_nodes.as<uint32_t>(),
+		t->top_links.as<uint2>(), t->level_end.as<uint32_t>(), info, t->root_box.as<SBox>(), room, t->health.as<uint32_t>());
 	return after_launch(ctx, "refit_top_kernel");
 }
 

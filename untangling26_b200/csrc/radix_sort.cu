@@ -655,12 +655,10 @@ namespace u26
 				radix_small_kernel<256><<<1, 256, sizeof(SmallSort<256>), ctx->stream>>>(keys, vals, n, bit_lo, bit_hi);
 			else
 			{
-				static std::atomic<bool> sized[64];
-				if (ctx->device < 0 || ctx->device >= 64 || !sized[ctx->device].load(std::memory_order_acquire))
+				if (!ctx->sized_sort.load(std::memory_order_acquire))
 				{
 					U26_CUDA(ctx, cudaFuncSetAttribute(radix_small_kernel<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SmallSort<1024>))));
-					if (ctx->device >= 0 && ctx->device < 64)
-						sized[ctx->device].store(true, std::memory_order_release);
+					ctx->sized_sort.store(true, std::memory_order_release);
 				}
 				radix_small_kernel<1024><<<1, 1024, sizeof(SmallSort<1024>), ctx->stream>>>(keys, vals, n, bit_lo, bit_hi);
 			}

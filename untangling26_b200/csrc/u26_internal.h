@@ -23,6 +23,9 @@ struct u26_ctx
 	// device address of the allocation-free EF sort's static scratch, looked up by the first
 	// u26_ef_canonicalize_noalloc call on this context
 	unsigned char* noalloc_scratch = nullptr;
+	// kernels whose dynamic shared memory limit this context has raised (a context made after a device reset
+	// raises it anew); several threads may raise it at once
+	std::atomic<bool> sized_plan{ false }, sized_sort{ false };
 };
 
 namespace u26
