@@ -539,7 +539,7 @@ def main():
         if r.device_error_flags:
             raise SystemExit(f"device error flags 0x{r.device_error_flags:x}")
         # every timed pass returns the same results (the leaf-test count may differ by a few between
-        # passes: see the packet walk's node tests)
+        # passes)
         if not wl.repair and (r.results.tobytes() != r0.results.tobytes() or any(a.tobytes() != b.tobytes() for a, b in zip(r.hits, r0.hits))):
             raise SystemExit("timed passes returned different results")
     repair = None

@@ -241,7 +241,7 @@ typedef struct u26_prp_params
 								 * selected direction on S^2 (intersection_resolver2.cpp:1232-1486) */
 	uint32_t ccr_blend;			/* PRP_use_blended_intrinsic_coordinates (0): one blended ownership coordinate */
 	float ccr_blend_weight;		/* PRP_intrinsic_blend_weight (0.5): rest-coordinate weight of the blend */
-	uint32_t form;				/* ray casting form: 0 batched packet traversal clipped to the candidate boxes (default),
+	uint32_t form;				/* ray casting form: 0 batched per-ray walk clipped to the candidate boxes (default),
 								 * 1 the plain form (one thread per request from the root, one launch per contour);
 								 * both decide the same pairs and return the same results */
 	uint32_t solid_interior;	/* PRP_solid_interior_adjacency (1): link hits through solid interiors */
@@ -257,7 +257,7 @@ typedef struct u26_prp_params
 								 * decisions. Also evaluates the selected supports' metrics in FP64 (fp64_*_rel_err). */
 	uint32_t autotune;			/* 1: the scene's first pass times every ray-casting configuration (subtree parts x blocks
 								 * per SM x grid form) on each of its launches and the scene keeps the fastest;
-								 * 0: 8 parts, 7 blocks, a warp per work item */
+								 * 0: 8 parts (4 in launches of 2^20 requests or more), 5 blocks, a work queue */
 	uint32_t raycast_config;	/* 0: the default or autotuned configuration; k in 1..18: use configuration k - 1 of the
 								 * table in u26_prp_output_view.tune_ms (every configuration returns the same results) */
 } u26_prp_params;
@@ -311,9 +311,9 @@ typedef struct u26_prp_output_view
 	uint64_t ray_nodes;				 /* ray / node box tests of the ray casts (per ray) */
 	uint64_t ray_edge_tests;		 /* leaf tests of the EE (edge-edge) casts, included in ray_tests */
 	double gpu_ms[6];				 /* GPU time (CUDA events): ray casting, hit sort, union-find, support entries, selection + metrics, download */
-	uint64_t ray_node_fetches;		 /* BVH node records brought in by the ray casts (one per warp packet visit) */
-	uint64_t ray_tri_fetches;		 /* triangle leaf records brought in (one per packet leaf visit) */
-	uint64_t ray_edge_fetches;		 /* edge leaf records brought in */
+	uint64_t ray_node_fetches;		 /* BVH node records read by the rays' walks (one per node a ray tests) */
+	uint64_t ray_tri_fetches;		 /* triangle leaf records read */
+	uint64_t ray_edge_fetches;		 /* edge leaf records read */
 	uint64_t ray_visits;			 /* BVH node tests each ray alone would make (the per-ray traversal work) */
 	uint64_t ray_candidate_tests;	 /* leaf tests whose primitive is a candidate target of the request's task */
 	uint64_t fp64_rechecks;			 /* with fp64_recheck: leaf tests inside their FP32 error band, re-evaluated in FP64 */

@@ -632,7 +632,7 @@ namespace u26
 
 		// ------------------------------------------------------------ request order
 		// Candidate vertices / edges of each slot ordered by the Morton code of their rest
-		// position (edge midpoint), so that the 32 requests of a warp packet start from a
+		// position (edge midpoint), so that a warp's 32 requests start from a
 		// compact patch. Only the request order changes: hits are keyed by primitive ids.
 		// Dense request-order ranks, made once per scene: the position of each vertex (edge) in
 		// the order of (Morton code, id). Candidates keyed by (slot, rank) sort into the
@@ -670,8 +670,8 @@ namespace u26
 					hi = mid;
 			}
 			const uint32_t id = cand[size_t(slot_ids[lo]) * stride + (g - off[lo])];
-			// (slot, dense rank of (Morton code, id)): unique keys, so the request order (and the
-			// packets) do not depend on the order the candidates were found in
+			// (slot, dense rank of (Morton code, id)): unique keys, so the request order does
+			// not depend on the order the candidates were found in
 			keys[g] = (uint64_t(lo) << id_bits) | rank[id];
 			vals[g] = id;
 		}

@@ -25,7 +25,7 @@ class PrpParams(ctypes.Structure):
         ("opt_iterations", c_u32),    # PRP_direction_optimization_iterations (0 = off)
         ("ccr_blend", c_u32),         # PRP_use_blended_intrinsic_coordinates
         ("ccr_blend_weight", c_f32),  # PRP_intrinsic_blend_weight
-        ("form", c_u32),              # 0 batched packet ray casting (default), 1 plain form (baseline)
+        ("form", c_u32),              # 0 batched ray casting (default), 1 plain form (baseline)
         ("solid_interior", c_u32),    # PRP_solid_interior_adjacency
         ("solid_all", c_u32),         # PRP_solid_interior_adjacency_all_meshes
         ("solid_eps_n", c_f32),       # PRP_solid_interior_adjacency_normal_eps
