@@ -1444,8 +1444,13 @@ namespace u26
 				W.u[5][lane] = plane ? 1u : 0u, W.u[6][lane] = ev.x, W.u[7][lane] = ev.y;
 				__syncwarp();
 				const uint32_t tested0 = tested;
-				const f3 sc = 0.5f * (smn + smx), sh = 0.5f * (smx - smn);
-				const float proj_c = 0.5f * (proj_lo + proj_hi), proj_h = 0.5f * (proj_hi - proj_lo);
+				// Centres and half extents of the swept box and of its extent along dir. The box test below rounds
+				// them three times more than it rounds the bounds themselves, each time by at most 2^-24 of the larger
+				// bound, which the node's margin does not cover when the swept edge is some hundred times longer
+				// than the node's distance from the origin: the half extents are widened by 2^-22 of it.
+				auto half = [](float lo, float hi) { return 0.5f * (hi - lo) + 0x1p-22f * fmaxf(fabsf(lo), fabsf(hi)); };
+				const f3 sc = 0.5f * (smn + smx), sh = mk3(half(smn.x, smx.x), half(smn.y, smx.y), half(smn.z, smx.z));
+				const float proj_c = 0.5f * (proj_lo + proj_hi), proj_h = half(proj_lo, proj_hi);
 				const f3 wn = plane ? pn : mk3(0.0f); // (no plane: every box meets the slab)
 				const float wd = plane ? pd : 0.0f;
 				ray_walk(
@@ -1454,8 +1459,9 @@ namespace u26
 					// swept edge's (a box that misses it holds no edge the swept edge reaches); and it meets the
 					// slab |dot(pn, q) - pd| <= 1e-6 around the swept edge's plane (a box clear of it holds only
 					// edges the leaf's separating-plane test rejects; cached_bvh.cpp:433-473 prunes its nodes the same
-					// way). Explicit fmas: the boxes carry the 1e-5 (1 + |c|) margin, far above this
-					// test's rounding, so no edge the leaf test keeps is pruned.
+					// way). Explicit fmas: the boxes carry the 1e-5 (1 + |c|) margin, far above the rounding of
+					// the node's own terms, and the swept extents carry theirs, so no edge that the tests on
+					// the bounds themselves would keep is pruned.
 					[&](const NodeBox& g)
 					{
 						const float cp = __fmaf_rn(g.mn.z, dir.z, __fmaf_rn(g.mn.y, dir.y, g.mn.x * dir.x));
