@@ -11,14 +11,17 @@
 // 3.9 M edges, 0.122 ms against 0.087 ms on 24,066.)
 //
 // Visit order, the 32-entry stack and the 100,000 step bound are the reference's, per query: a query whose
-// stack is full stops and raises the flag. With split > 1 (parts of the tree below its first
-// levels, for query sets too small to fill the chip) a part does not see another part's stop.
+// stack is full, or that has taken its steps, stops and raises the flag; what it met before counts.
+// Query sets too small to fill the chip are split into the parts of the tree below its first levels, where
+// neither bound can be met (walk_split_log2, walk_part), since a part would not see another part's stop.
 #pragma once
 #include "lbvh_internal.h"
 
 namespace u26
 {
-	constexpr uint32_t kLeafQueue = 128; // 31 left over + 2 x 32 new entries at most
+	constexpr uint32_t kLeafDrain = 64; // entries from which the queue is emptied to a batch's rest
+	constexpr uint32_t kLeafQueue = 128;
+	static_assert(kLeafDrain - 1 + 2 * 32 <= kLeafQueue, "a step adds two leaves a lane to a queue below the drain mark");
 	constexpr uint32_t kQueryStack = 32;
 	constexpr uint32_t kQuerySteps = 100000u;
 
@@ -29,14 +32,27 @@ namespace u26
 	};
 
 	// Parts per query warp: doubled until 64 warps per SM are there, at most 32 (24,066 edges in 16 parts:
-	// 0.087 ms; four times as many warps 0.094 ms).
-	inline uint32_t walk_split_log2(uint32_t num_queries)
+	// 0.087 ms; four times as many warps 0.094 ms). One part when the tree has more inner nodes than a query may
+	// take steps.
+	inline uint32_t walk_split_log2(uint32_t num_queries, uint32_t num_leaves)
 	{
 		const uint32_t warps = div_up(num_queries, 32);
 		uint32_t s = 0;
-		while (s < 5 && (uint64_t(warps) << s) < 148u * 64u)
-			s++;
+		if (num_leaves <= kQuerySteps + 1u)
+			while (s < 5 && (uint64_t(warps) << s) < 148u * 64u)
+				s++;
 		return s;
+	}
+	// The depth of this part's split, known on the device only; false when the part has no walk. A node whose
+	// two children are stacked lies at most height - 2 below the root, and each node above it holds
+	// at most one entry: a tree of height 32 never fills the stack. (Meshes of 100,000 triangles are 20 to 30 high;
+	// several scenes in one tree up to 40.)
+	__device__ __forceinline__ bool walk_part(const TreeView& tv, uint32_t part, uint32_t& split_log2)
+	{
+		if (__ldg(tv.height) <= kQueryStack)
+			return true;
+		split_log2 = 0u;
+		return part == 0u;
 	}
 
 	// accept(prim): per lane, whether the leaf counts. flush(prim, lane, n): all lanes call it; lane k < n
@@ -86,18 +102,14 @@ namespace u26
 		// the start: the root, or the part's node below the first levels
 		uint2 cur = __ldg(tv.children); // the children of the node that the lane stands at
 		bool on = valid;
-		uint32_t limit = kQueryStack; // entries that this part may stack
 		for (uint32_t l = split_log2; l > 0 && __any_sync(kAll, on); l--)
 		{
 			const bool right = (part >> (l - 1)) & 1u;
 			const bool mine = (part & ((1u << (l - 1)) - 1u)) == 0u; // the part that counts this step
-			const uint32_t c = right ? cur.y : cur.x, o = right ? cur.x : cur.y;
+			const uint32_t c = right ? cur.y : cur.x;
 			const bool hit = on && meets(c);
 			visited += on && mine ? 1u : 0u;
 			const uint2 next = __ldg(tv.children + c);
-			// the first child waits on the query's stack while the second's subtree is walked
-			if (right && o < ni && on && meets(o))
-				limit--;
 			on = hit;
 			if (c >= ni) // (uniform)
 			{
@@ -124,13 +136,13 @@ namespace u26
 			}
 			const bool leaf_x = cur.x >= ni, leaf_y = cur.y >= ni;
 			bool go_x = hx && !leaf_x, go_y = hy && !leaf_y;
-			if (go_x && top >= limit)
+			if (go_x && top >= kQueryStack)
 			{
 				atomicOr(dev_err, U26_DEVERR_STACK_OVERFLOW);
 				go_x = go_y = hy = on = false;
 				visited--; // the second child is not tested
 			}
-			else if (go_y && top + (go_x ? 1u : 0u) >= limit)
+			else if (go_y && top + (go_x ? 1u : 0u) >= kQueryStack)
 			{
 				atomicOr(dev_err, U26_DEVERR_STACK_OVERFLOW);
 				go_x = go_y = on = false;
@@ -158,7 +170,7 @@ namespace u26
 				else
 					on = false;
 			}
-			if (count >= 64u)
+			if (count >= kLeafDrain)
 				drain(31u);
 		}
 		drain(0u);

@@ -207,6 +207,8 @@ namespace u26
 			if (wi >= uint64_t(warps) << split_log2 || *tv.health == 0u)
 				return;
 			const uint32_t part = uint32_t(wi / warps), q0 = uint32_t(wi - uint64_t(part) * warps) * 32u;
+			if (!walk_part(tv, part, split_log2))
+				return;
 			const bool valid = q0 + lane < num_edges;
 			const uint32_t tid = valid ? q0 + lane : num_edges - 1u;
 			f3 mn, mx;
@@ -547,7 +549,7 @@ U26_API u26_status u26_ef_detect(u26_lbvh* face_tree, const float* x, const uint
 		return set_error(ctx, U26_ERR_INVALID_INPUT, "u26_ef_detect: null input");
 	if (num_edges == 0)
 		return U26_OK;
-	const uint32_t split = walk_split_log2(num_edges);
+	const uint32_t split = walk_split_log2(num_edges, face_tree->n);
 	const uint32_t grid = uint32_t(div_up64(uint64_t(div_up(num_edges, 32)) << split, 4));
 	auto launch = [&](auto* kernel)
 	{

@@ -575,7 +575,7 @@ namespace u26
 		constexpr uint32_t kChunkThreads = 512;
 		__global__ void __launch_bounds__(kChunkThreads) plan_words_kernel(const uint32_t* __restrict__ parent, const uint2* __restrict__ children,
 			const uint32_t* __restrict__ node_range, uint32_t n, const uint32_t* __restrict__ chunk_lo, const uint32_t* __restrict__ chunk_tb,
-			const uint32_t* __restrict__ info, const uint32_t* __restrict__ roots, uint32_t* __restrict__ words, uint8_t* __restrict__ root_height,
+			uint32_t* __restrict__ info, const uint32_t* __restrict__ roots, uint32_t* __restrict__ words, uint8_t* __restrict__ root_height,
 			uint32_t* __restrict__ health)
 		{
 			__shared__ uint32_t s_word[kTreelet], s_parent[kTreelet], s_leaf_parent[kTreelet], s_count[kTreelet];
@@ -654,6 +654,8 @@ namespace u26
 				const uint32_t x = roots[b];
 				const uint32_t k = x >= ni ? x - ni - base : x - base;
 				root_height[b] = x < ni && k < cnt ? s_height[k] : uint8_t(0);
+				if (x == 0u && k < cnt)
+					info[3] = s_height[k]; // the tree's root
 				if (k >= cnt)
 					atomicExch(health, 0u);
 			}
@@ -666,7 +668,7 @@ namespace u26
 		};
 		constexpr uint32_t kTopScratchShared = 12u * 1024u; // top nodes whose scratch fits in shared memory (192 KB)
 		__global__ void __launch_bounds__(1024) plan_top_kernel(Plan plan, const uint32_t* __restrict__ parent, const uint2* __restrict__ children,
-			const uint32_t* __restrict__ info, const uint8_t* __restrict__ root_height, TopScratch* __restrict__ scratch,
+			uint32_t* __restrict__ info, const uint8_t* __restrict__ root_height, TopScratch* __restrict__ scratch,
 			uint32_t* __restrict__ top_nodes, uint2* __restrict__ top_links, uint32_t* __restrict__ root_slot,
 			uint32_t* __restrict__ level_end, uint32_t* __restrict__ health)
 		{
@@ -736,6 +738,8 @@ namespace u26
 					root_slot[min(r, nt - 1u)] = 2u * place + side;
 					return kTopRoot | r;
 				};
+				if (S[j].parent == kInvalid)
+					info[3] = S[j].height; // the tree's root
 				const uint2 raw = plan.top_raw[j];
 				top_links[place] = make_uint2(compact(raw.x, 0u), compact(raw.y, 1u));
 				top_nodes[S[j].place] = plan.top_list[j];
@@ -1000,6 +1004,8 @@ namespace u26
 			if (wi >= uint64_t(warps) << split_log2 || *tv.health == 0u)
 				return;
 			const uint32_t part = uint32_t(wi / warps), q0 = uint32_t(wi - uint64_t(part) * warps) * 32u;
+			if (!walk_part(tv, part, split_log2))
+				return;
 			const bool valid = q0 + lane < nq;
 			const uint32_t q = valid ? q0 + lane : nq - 1u;
 			f3 mn, mx;
@@ -1360,7 +1366,7 @@ U26_API u26_status u26_lbvh_query(u26_lbvh* t, int mode, const float* x_begin, c
 		return U26_OK;
 	u26_ctx* ctx = t->ctx;
 	const TreeView tv = tree_view(t);
-	const uint32_t split = walk_split_log2(num_queries);
+	const uint32_t split = walk_split_log2(num_queries, t->n);
 	const uint32_t grid = uint32_t(div_up64(uint64_t(div_up(num_queries, 32)) << split, 4));
 	if (mode == U26_QUERY_VERTS)
 		query_kernel<U26_QUERY_VERTS><<<grid, 128, 0, ctx->stream>>>(tv, x_begin, x_end, edges, num_queries, d_hat, thickness, count,

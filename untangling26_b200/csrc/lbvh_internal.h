@@ -31,7 +31,7 @@ struct u26_lbvh
 	// refit plan, prepared by construct_tree (one per topology; its counts stay on the device): parts of one
 	// allocation
 	u26::DevBuf plan;
-	u26::DevView plan_info;		 // uint32[4]: top nodes m, treelets nt, chunks
+	u26::DevView plan_info;		 // uint32[4]: top nodes m, treelets nt, chunks, the tree's height (leaves 0)
 	u26::DevView plan_words;		 // uint32[max(n-1,1)]: chunk-local child slots and height of each inner node
 	u26::DevView chunk_lo;		 // uint32[chunks + 1]: first leaf of each refit chunk, then n
 	u26::DevView chunk_tb;		 // uint32[chunks + 1]: first treelet of each chunk, then nt
@@ -70,11 +70,12 @@ namespace u26
 		const uint2* __restrict__ children;
 		const uint32_t* __restrict__ object_idx;
 		const uint32_t* __restrict__ health;
+		const uint32_t* __restrict__ height;
 		uint32_t n;
 	};
 	inline TreeView tree_view(const u26_lbvh* t)
 	{
 		return TreeView{ t->node_aabb.as<NodeBox>(), t->children.as<uint2>(), t->object_idx.as<uint32_t>(),
-			t->health.as<uint32_t>(), t->n };
+			t->health.as<uint32_t>(), t->plan_info.as<uint32_t>() + 3, t->n };
 	}
 } // namespace u26
