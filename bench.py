@@ -538,8 +538,7 @@ def main():
     for r in results:
         if r.device_error_flags:
             raise SystemExit(f"device error flags 0x{r.device_error_flags:x}")
-        # every timed pass returns the same results (the leaf-test count may differ by a few between
-        # passes)
+        # every timed pass returns the same results
         if not wl.repair and (r.results.tobytes() != r0.results.tobytes() or any(a.tobytes() != b.tobytes() for a, b in zip(r.hits, r0.hits))):
             raise SystemExit("timed passes returned different results")
     repair = None
@@ -599,7 +598,7 @@ def main():
         from untangling26_b200.prp import config_name
         mine = config_name((r0.raycast_config["parts"], r0.raycast_config["blocks_per_sm"], r0.raycast_config["queue"]))
         roof["traffic_config"] = {"captured": tr.get("raycast_config"), "this_run": mine, "same": tr.get("raycast_config") == mine}
-    roof["packet_record_bytes_per_pass"] = 32 * r0.node_fetches + 48 * r0.tri_fetches + 32 * r0.edge_fetches + 24 * r0.requests
+    roof["record_bytes_per_pass"] = 32 * r0.node_fetches + 48 * r0.tri_fetches + 32 * r0.edge_fetches + 24 * r0.requests
 
     # ---- LBVH refit alone (fused leaf update + bottom-up refit of a face tree), L2 flushed
     # before each launch: the timed batch's scene tree and the scale form's mesh (five stacked

@@ -311,10 +311,10 @@ typedef struct u26_prp_output_view
 	uint64_t ray_nodes;				 /* ray / node box tests of the ray casts (per ray) */
 	uint64_t ray_edge_tests;		 /* leaf tests of the EE (edge-edge) casts, included in ray_tests */
 	double gpu_ms[6];				 /* GPU time (CUDA events): ray casting, hit sort, union-find, support entries, selection + metrics, download */
-	uint64_t ray_node_fetches;		 /* BVH node records read by the rays' walks (one per node a ray tests) */
-	uint64_t ray_tri_fetches;		 /* triangle leaf records read */
-	uint64_t ray_edge_fetches;		 /* edge leaf records read */
-	uint64_t ray_visits;			 /* BVH node tests each ray alone would make (the per-ray traversal work) */
+	uint64_t ray_node_fetches;		 /* BVH node records read by the rays' walks (a record per test: ray_nodes) */
+	uint64_t ray_tri_fetches;		 /* triangle leaf records read (ray_tests - ray_edge_tests) */
+	uint64_t ray_edge_fetches;		 /* edge leaf records read (ray_edge_tests) */
+	uint64_t ray_visits;			 /* BVH node tests each ray alone would make: ray_nodes, since every ray walks alone */
 	uint64_t ray_candidate_tests;	 /* leaf tests whose primitive is a candidate target of the request's task */
 	uint64_t fp64_rechecks;			 /* with fp64_recheck: leaf tests inside their FP32 error band, re-evaluated in FP64 */
 	uint64_t fp64_flips;			 /* ... of which the FP64 decision differs from the FP32 one (the hit sets keep FP32) */
@@ -325,8 +325,8 @@ typedef struct u26_prp_output_view
 	double fp64_dc_rel_err;			 /* max over processed contours of |D_C,32 - D_C,64| / D_C,64 (depth) */
 	double fp64_j_rel_err;			 /* max over processed contours of |J_32 - J_64| / J_64 (objective) */
 	double tune_ms[18];				 /* autotune pass: ray-casting time (ms, summed over the pass's launches) of each
-									  * configuration (subtree parts, blocks per SM, grid form): (4,6) (4,7) (4,8) (8,6)
-									  * (8,7) (8,8) (16,6) (16,7) (16,8) with a warp per work item, then the same nine
+									  * configuration (subtree parts, blocks per SM, grid form): (4,4) (4,5) (4,6) (8,4)
+									  * (8,5) (8,6) (16,4) (16,5) (16,6) with a warp per work item, then the same nine
 									  * with a persistent grid whose warps take work items from a queue */
 	uint32_t raycast_parts;			 /* configuration the scene's ray casts use from now on: subtree parts per request (the
 									   * default's 8 are 4 in launches of 2^20 requests and more) */
@@ -455,7 +455,9 @@ U26_API u26_status u26_filter_broad_phase_pairs(u26_ctx* ctx, uint32_t* vf_list,
  * first). J's subgradient runs through the first maximal hit in key order. All pointers are
  * device memory: x [V][3], hits as u26_prp_resolve returns them, hit_offsets [C+1], dirs,
  * grad_dirs [C][3], the per-vertex / edge / face rest areas and vertex masses of the mesh;
- * J, E may be NULL. Runs on ctx's stream. */
+ * J, E may be NULL. Runs on ctx's stream. J, E and grad_dirs are the same on every call with the
+ * same inputs; the additions into grad_x are float atomics in no fixed order, also within one
+ * contour, so its last bits may differ. */
 U26_API u26_status u26_prp_adjoint(u26_ctx* ctx, const float* x, const u26_prp_hit* hits, const uint32_t* hit_offsets,
 	uint32_t num_contours, const float* dirs, const float* vert_area, const float* edge_area, const float* face_area,
 	const float* vert_mass, float* J, float* E, const float* grad_J, const float* grad_E, float* grad_dirs, float* grad_x);

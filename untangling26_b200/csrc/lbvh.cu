@@ -3,9 +3,9 @@
 // Reference: Solver/CollisionDetector/lbvh.cpp. Construction: global AABB
 // (372-452, 454-496, 988-1021), Morton keys (84-135, 512-528), sort (1037-1040, here a
 // device radix sort), Karras emission (206-293, 546-601), check (603-616). Refit:
-// leaf AABBs (621-688) and the bottom-up union (694-758), here with a per-node arrival
-// counter instead of the reference's float-CAS flags and spin-waits: the second thread
-// to reach a node owns it, so no thread ever waits on another. Query: stack-32
+// leaf AABBs (621-688) and the bottom-up union (694-758), here height by height from a plan
+// that construction prepares, instead of the reference's float-CAS flags and spin-waits: no
+// thread waits on another outside its block's barriers. Query: stack-32
 // traversal with strict overlap (295-363, 780-894), in the reference's visit order so
 // that the stack-overflow cut-off drops the same pairs.
 #include <algorithm>
@@ -399,19 +399,19 @@ namespace u26
 		//    64-bit keys is at most 64 deep);
 		//  * the top nodes (more than kTreelet leaves) sorted by height, their children as
 		//    compact ids (top node j, or 0x80000000 | treelet b).
-		// refit_chunk_kernel: one block per chunk. Leaf boxes, the chunk's inner nodes' words
-		// and their boxes live in shared memory; the nodes of height h are
+		// refit_chunk_kernel: one block per chunk. Leaf boxes and the chunk's inner nodes'
+		// boxes live in shared memory, the nodes' words in registers; the nodes of height h are
 		// united in step h, after a barrier, so every union reads finished children without
 		// atomics or fences. Boxes go out coalesced.
 		// refit_top_kernel: one block for the top tree, height by height, in shared memory when
 		// it fits, else through L2.
 		// Unions keep the (first child, second child) operand order of the reference.
 		// The plan's counts stay on the device and its arrays have their upper bounds' sizes from
-		// the start, so a construction is 9 to 14 launches without an allocation or a host read (heights by
+		// the start, so a construction is 5 to 10 kernels (4 of them in the sort of more than 8,192 keys) without an allocation or a host read (heights by
 		// device atomics over the whole tree, two sorts and two host reads made it 53 to 61). Face and edge
 		// tree constructed and refit: 3,844 triangles 1.80 ms, 0.18 ms now (host and launch latency); 130,050
 		// 1.85 ms, 0.29 ms; 2.6 M 3.5 ms, 1.45 ms (0.43 ms of it the sorts, 0.31 ms the one-block kernels).
-		constexpr size_t kChunkSmem = 2 * 24 * kTreelet + sizeof(uint32_t) * kTreelet;
+		constexpr size_t kChunkSmem = 2 * 24 * kTreelet;
 
 		// Top nodes lie above nodes of more than kTreelet leaves, disjoint at every depth, and a tree over
 		// 30 Morton bits and the leaf id bits has at most 62 depths with one: at most 62 n / 1025 < n / 16
@@ -779,8 +779,7 @@ namespace u26
 			const uint32_t* __restrict__ chunk_tb, const uint32_t* __restrict__ roots, const uint32_t* __restrict__ root_slot,
 			SBox* __restrict__ root_box, uint32_t* __restrict__ health)
 		{
-			// dynamic shared memory (kChunkSmem bytes, four blocks per SM): leaf boxes, inner boxes,
-			// the nodes' words
+			// dynamic shared memory (kChunkSmem bytes, four blocks per SM): leaf boxes, inner boxes
 			extern __shared__ __align__(16) unsigned char s_raw[];
 			SBox* s_leaf = reinterpret_cast<SBox*>(s_raw);
 			SBox* s_inner = s_leaf + kTreelet;

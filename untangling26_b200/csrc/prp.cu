@@ -196,9 +196,11 @@ namespace u26
 		// a queued bit for the relaxation: 4.125 B per vertex, up to kSharedVerts vertices); otherwise
 		// in global memory. Bound by the rounds' dependent accesses (45 BFS levels and about as many
 		// relaxation rounds on a 64 x 64 sheet): 0.95 ms with one
-		// 256-thread CTA and L2 atomics, 0.29 ms.
+		// 256-thread CTA and L2 atomics, 0.29 ms. Every block, also the BFS's, is given the largest object's state, so beside
+		// an object of 50,000 vertices one block has an SM; the stage is still the shorter one (64 pairs of 20 x 20 sheets
+		// and one of 228 x 228: 5.3 ms with the L2 form, 3.4 ms; 200 pairs of 16 x 16 and the large one: 6.8, 5.4).
 		constexpr uint32_t kDistThreads = 512;
-		constexpr uint32_t kSharedVerts = 53000; // 218,625 bytes
+		constexpr uint32_t kSharedVerts = 53000; // 218,628 bytes
 		inline size_t dist_smem(uint32_t verts) { return 4u * size_t(verts) + 4u * size_t(verts / 32u + 1u); }
 		template <bool SHARED>
 		__global__ void __launch_bounds__(kDistThreads) distances_kernel(Slot* __restrict__ slots, const uint32_t* __restrict__ slot_ids,
@@ -984,12 +986,14 @@ namespace u26
 		// ms, 10.2 ms. Measured and dropped: records of four grandchildren (half the dependent steps; 121 ms where
 		// this took 113: the registers of four boxes in flight).
 		constexpr int kStack = 64;
+		constexpr uint32_t kRayDrain = 64, kRayQueue = 128; // leaf entries from which the queue is emptied, and its size
+		static_assert(kRayDrain - 1 + 2 * 32 <= kRayQueue, "a step adds two leaves a lane to a queue below the drain mark");
 		struct RayWarp
 		{
 			float f[14][32];	  // a ray's or swept edge's constants, by lane
 			uint32_t u[8][32];
-			uint32_t prim[128]; // leaf queue: 31 left over + 2 x 32 new entries at most
-			uint8_t from[128];
+			uint32_t prim[kRayQueue]; // leaf queue
+			uint8_t from[kRayQueue];
 		};
 		__device__ __forceinline__ NodeBox load_node(const NodeBox* p)
 		{
@@ -1246,7 +1250,7 @@ namespace u26
 						atomicOr(dev_err, U26_DEVERR_ITERATION_CAP);
 					on = false;
 				}
-				if (count >= 64u)
+				if (count >= kRayDrain)
 					drain(31u);
 			}
 			drain(0u);
@@ -1524,9 +1528,13 @@ namespace u26
 		constexpr RaycastConfig kRaycastConfigs[] = { { 4, 4, false }, { 4, 5, false }, { 4, 6, false }, { 8, 4, false }, { 8, 5, false },
 			{ 8, 6, false }, { 16, 4, false }, { 16, 5, false }, { 16, 6, false }, { 4, 4, true }, { 4, 5, true }, { 4, 6, true }, { 8, 4, true },
 			{ 8, 5, true }, { 8, 6, true }, { 16, 4, true }, { 16, 5, true }, { 16, 6, true } };
-		// The default: the queue at 5 blocks per SM, in 8 parts. Parts share a ray's setup but not its balance: 16
-		// scenes of 2k-60k triangles take 102 ms in 4 parts, 111 in 8; a folded sheet with 26 directions 11.8, 10.1
-		// (9.4 in 16); two 64 x 64 sheets 5.6, 6.2. Launches of kManyRequests and more (the first kind) use 4.
+		// The default: the queue at 5 blocks per SM, in 8 parts, and in 4 for launches of kManyRequests and more. Parts share a
+		// ray's setup but not its balance, and what decides is the scene, not the number of requests: pairs of bodies
+		// take 4 at every size (ray casting of a pass in 4 / 8 / 16 parts: two 64 x 64 sheets 3.1 / 3.4 / 3.6 ms,
+		// 128 x 128 9.5 / 10.3 / 11.0, four scenes 14.2 / 15.5 / 17.1, sixteen 26.0 / 28.6 / 32.5), a sheet folded on itself
+		// 8 or 16 (64 x 64 3.5 / 2.9 / 2.7, with 26 directions 4.8 / 4.1 / 4.0, 128 x 128 25.2 / 20.2 / 18.1). 8 parts
+		// are within a sixth of the best of each (two sheets with 26 directions 6.0 / 6.9 / 8.6); large launches are
+		// mostly batches', and the autotuner finds a scene's own.
 		constexpr int kNumRaycastConfigs = 18, kDefaultRaycastConfig = 13;
 		constexpr uint32_t kManyRequests = 1u << 20;
 		using RaycastFn = decltype(&raycast_kernel<false, 5, false>);

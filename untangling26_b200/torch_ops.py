@@ -8,6 +8,8 @@ as delta = (w . n) / (r . n) on the supports S(r) of a u26_prp_resolve pass (hel
 function is the smooth branch of the objective around the pass). backward gives dJ/dx, dE/dx
 (dense [V, 3]) and dJ/dr, dE/dr through one hand-written adjoint kernel; dE/dr is the
 gradient the reference's direction refinement uses (intersection_resolver2.cpp:1268-1320).
+J, E and the gradients in the directions repeat bit for bit; those in the positions are summed by
+float atomics in no fixed order, so their last bits may differ between calls.
 There is no CPU path: the tensors live on the context's CUDA device.
 """
 import ctypes
