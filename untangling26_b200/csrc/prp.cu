@@ -2015,6 +2015,7 @@ namespace u26
 		}
 
 		constexpr uint32_t kFewHits = 1u << 18; // their table (8 MB) is cleared in the time of a launch
+		constexpr uint32_t kManyHits = 1u << 22; // terms of as many hits: 50 MB
 
 		// find_adjacent_hits rules as exact key lookups inside the task segment. Lookups that
 		// share a (type, source) first find that source's run of hits once, then search the
@@ -5101,16 +5102,17 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 			U26_TRY(after_launch(ctx, "sel_block_sums_kernel"));
 			scan_one_block_kernel<<<1, 1024, 0, st>>>(S->d_bsum.as<uint32_t>(), nblk, S->d_bsum.as<uint32_t>() + nblk + 1);
 			U26_TRY(after_launch(ctx, "scan_one_block_kernel"));
-			// (the number of selected hits is read back only where the hits are: the terms' buffer holds
-			// every hit's)
-			if (hits_out || trace)
+			// (the number of selected hits is read back only where the hits are, and in levels of so many hits that the
+			// terms' buffer should not hold every hit's)
+			nsel = nh;
+			if (hits_out || trace || nh > kManyHits)
 			{
 				U26_CUDA(ctx, cudaMemcpyAsync(ctx->host_word, S->d_bsum.as<uint32_t>() + nblk + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
 				U26_CUDA(ctx, cudaStreamSynchronize(st));
 				nsel = *ctx->host_word;
 			}
 			U26_CUDA(ctx, S->d_pos.reserve(sizeof(uint32_t) * nh1));
-			U26_CUDA(ctx, S->d_terms.reserve(sizeof(float) * 3 * size_t(nh1)));
+			U26_CUDA(ctx, S->d_terms.reserve(sizeof(float) * 3 * size_t(std::max(nsel, 1u))));
 			if (hits_out)
 				U26_CUDA(ctx, S->d_sel.reserve(sizeof(u26_prp_hit) * size_t(std::max(nsel, 1u))));
 			sel_terms_kernel<<<nblk, 256, 0, st>>>(S->d_keys.as<uint64_t>(), S->d_root.as<uint32_t>(), d_best, cd, nh, S->d_bsum.as<uint32_t>(),

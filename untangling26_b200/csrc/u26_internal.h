@@ -34,7 +34,9 @@ namespace u26
 	extern std::atomic<uint64_t> g_alloc_count;
 
 	// Grow-only device allocation owned by a context-side object. A buffer that grows takes half as much again as
-	// it held: a scene's first pass asks for more at every level, and each growth waits for the device.
+	// it held, at most kGrowSlack more than was asked for: a scene's first pass asks for more at every level, and each growth
+	// waits for the device; above that size the level's own work hides the wait, and the memory counts.
+	constexpr size_t kGrowSlack = size_t(32) << 20;
 	struct DevBuf
 	{
 		void* ptr = nullptr;
@@ -43,7 +45,7 @@ namespace u26
 		{
 			if (want <= bytes)
 				return cudaSuccess;
-			const size_t grown = std::max(want, bytes + bytes / 2);
+			const size_t grown = std::max(want, std::min(bytes + bytes / 2, want + kGrowSlack));
 			if (ptr)
 				cudaFree(ptr);
 			ptr = nullptr;
