@@ -55,3 +55,16 @@ def test_both_forms_agree_on_long_edges(u26ctx, length, axis, directions):
             assert a.tobytes() == b.tobytes()
         assert batched.results.tobytes() == plain.results.tobytes()
     assert u26ctx.device_errors() == 0
+
+
+@pytest.mark.parametrize("length, directions, seed, rechecks, flips", [
+    (1, 1, 0, 5560, 32), (300, 1, 1, 32352, 282), (1000, 0, 2, 7848, 36), (1000, 1, 1, 43429, 288), (4000, 0, 1, 19002, 21),
+    (4000, 1, 2, 49957, 149), (20000, 0, 2, 65730, 24), (20000, 1, 0, 187364, 183)])
+def test_recheck_counts_on_long_edges(u26ctx, length, directions, seed, rechecks, flips):
+    """The counted FP64 rechecks are those of the leaf tests that a walk testing the boxes' bounds themselves makes
+    (its counts are given), not of what the margins on centres and half extents add."""
+    sc = CollisionScene(u26ctx, _mesh(length, seed, 0))
+    sc.construct_lbvh()
+    res = sc.untangle_pass(prp_params(max_contours=64, direction_mode=directions, fp64_recheck=1))
+    sc.close()
+    assert (res.fp64["rechecks"], res.fp64["flips"]) == (rechecks, flips)

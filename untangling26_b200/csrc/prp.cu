@@ -785,6 +785,10 @@ namespace u26
 			return tmin <= tmax;
 		}
 
+		// Half of [lo, hi], and eight roundings (2^-21) of its larger bound: a test on centres and half extents (a sum, a
+		// difference and a fused dot product of each) keeps whatever the same test on the bounds themselves keeps.
+		__device__ __forceinline__ float half_extent(float lo, float hi) { return 0.5f * (hi - lo) + 0x1p-21f * fmaxf(fabsf(lo), fabsf(hi)); }
+
 		// Conservative node margins, applied to every node once per pass so that the traversals
 		// read grown boxes: eps = 1e-5 (1 + max |bound|) per axis for the ray slab tests, one eps
 		// from all six bounds for the swept-edge box tests (the epsilon-grown node tests that
@@ -805,12 +809,13 @@ namespace u26
 			if (isotropic)
 			{
 				const float e = 1e-5f * (1.0f + fmaxf(fmaxf(fabsf(b.mn.x), fabsf(b.mx.x)), fmaxf(fmaxf(fabsf(b.mn.y), fabsf(b.mx.y)), fmaxf(fabsf(b.mn.z), fabsf(b.mx.z)))));
-				// centre and half extents, as the swept-edge box test takes them; an axis with an infinite or NaN
-				// bound covers everything (the exact tests decide)
+				// centre and half extents, as the swept-edge box test takes them, the half extents with that test's
+				// rounding of the node's terms (half_extent); an axis with an infinite or NaN bound covers everything (the
+				// exact tests decide)
 				auto axis = [&](float lo, float hi, float& c, float& h)
 				{
 					c = 0.5f * (lo + hi);
-					h = 0.5f * (hi - lo);
+					h = half_extent(lo, hi);
 					if (!isfinite(c) || !isfinite(h))
 					{
 						c = 0.0f;
@@ -1013,9 +1018,59 @@ namespace u26
 			const uint32_t *bits_e, *bits_f;
 			uint32_t e_words, f_words; // bitmap words per slot
 			HitSink sink;
+			const float* slot_box; // [slots][12]
+			const Task* tasks;
 		};
 		extern __shared__ __align__(16) unsigned char s_ray_raw[]; // RayWarp per warp
 		__device__ __forceinline__ RayWarp& ray_warp() { return reinterpret_cast<RayWarp*>(s_ray_raw)[threadIdx.x >> 5]; }
+
+		// A swept edge's extent along dir (prp_compute_edge_projection_bounds with the target edges' lower bound,
+		// cached_bvh.cpp:377-473), widened by 1e-6, and its box, clipped to the grown AABB tb of the candidate target edges.
+		__device__ __forceinline__ void swept_extent(f3 p0, f3 p1, f3 dir, float dl2, float ray_max, float ee_pmin, float& lo, float& hi)
+		{
+			const float ep0 = dot(p0, dir), ep1 = dot(p1, dir);
+			lo = fmaxf(fminf(ep0, ep1), ee_pmin - 1e-5f) - 1e-6f;
+			hi = (fmaxf(ep0, ep1) + ray_max * dl2) + 1e-6f;
+		}
+		__device__ __forceinline__ void swept_box(f3 p0, f3 p1, f3 dir, float ray_max, const float* __restrict__ tb, f3& mn, f3& mx)
+		{
+			const f3 a_end = p0 + dir * ray_max, b_end = p1 + dir * ray_max;
+			const float g0 = 1e-5f * (1.0f + fmaxf(fabsf(tb[0]), fabsf(tb[3])));
+			const float g1 = 1e-5f * (1.0f + fmaxf(fabsf(tb[1]), fabsf(tb[4])));
+			const float g2 = 1e-5f * (1.0f + fmaxf(fabsf(tb[2]), fabsf(tb[5])));
+			mn = vmax(vmin(vmin(p0, p1), vmin(a_end, b_end)), mk3(tb[0] - g0, tb[1] - g1, tb[2] - g2));
+			mx = vmin(vmax(vmax(p0, p1), vmax(a_end, b_end)), mk3(tb[3] + g0, tb[4] + g1, tb[5] + g2));
+		}
+		// Whether the swept edge of lane `from` meets the grown box of the edge (q0, q1) by the tests on the bounds
+		// themselves: the leaf tests whose FP64 rechecks count (the walk reaches these and, by its margins, a few more).
+		// Out of line: one lane in 250 asks.
+		__device__ __noinline__ bool edge_reached(const LeafArgs& L, uint32_t from, f3 q0, f3 q1)
+		{
+			const RayWarp& W = ray_warp();
+			const f3 p0 = mk3(W.f[0][from], W.f[1][from], W.f[2][from]), p1 = ld3(L.x, W.u[7][from]);
+			const f3 dir = mk3(W.f[6][from], W.f[7][from], W.f[8][from]), pn = mk3(W.f[9][from], W.f[10][from], W.f[11][from]);
+			const float pd = W.f[12][from], ray_max = W.f[13][from];
+			f3 smn, smx;
+			float proj_lo, proj_hi;
+			swept_box(p0, p1, dir, ray_max, L.slot_box + 12 * size_t(W.u[2][from]) + 6, smn, smx);
+			swept_extent(p0, p1, dir, dot(dir, dir), ray_max, L.tasks[W.u[1][from]].ee_pmin, proj_lo, proj_hi);
+			f3 mn = vmin(q0, q1), mx = vmax(q0, q1);
+			const float e = 1e-5f * (1.0f + fmaxf(fmaxf(fabsf(mn.x), fabsf(mx.x)), fmaxf(fmaxf(fabsf(mn.y), fabsf(mx.y)), fmaxf(fabsf(mn.z), fabsf(mx.z)))));
+			mn = mn - mk3(e);
+			mx = mx + mk3(e);
+			if (!((smn.x <= mx.x) & (smx.x >= mn.x) & (smn.y <= mx.y) & (smx.y >= mn.y) & (smn.z <= mx.z) & (smx.z >= mn.z)))
+				return false;
+			const f3 c = mk3(0.5f * (mn.x + mx.x), 0.5f * (mn.y + mx.y), 0.5f * (mn.z + mx.z));
+			const f3 h = mk3(0.5f * (mx.x - mn.x), 0.5f * (mx.y - mn.y), 0.5f * (mx.z - mn.z));
+			const float cp = dot(c, dir);
+			const float pr = (h.x * fabsf(dir.x) + h.y * fabsf(dir.y)) + h.z * fabsf(dir.z);
+			if (cp + pr < proj_lo || cp - pr > proj_hi)
+				return false;
+			if (W.u[5][from] == 0u)
+				return true;
+			const float rad = (h.x * fabsf(pn.x) + h.y * fabsf(pn.y)) + h.z * fabsf(pn.z);
+			return fabsf(dot(pn, c) - pd) <= rad + 1e-6f;
+		}
 
 		// 32 leaf tests, entry (primitive, lane) k < n in lane k. Out of line: one call per 32 tests, and the walk
 		// keeps its registers. Returns 1 when the entry's primitive is a candidate, plus its FP64 recheck (256) and
@@ -1138,7 +1193,7 @@ namespace u26
 					Band bd;
 					if (RECHECK)
 						edge_edge_band(p0, e1, dir, ray_max, plane, pn, pd, q0, q1, bd);
-					if (RECHECK && bd.recheck())
+					if (RECHECK && bd.recheck() && edge_reached(L, from, q0, q1))
 					{
 						const uint32_t rc = recheck_ee(p0, e1, dir, ray_max, q0, q1, ee_hit);
 						told += (rc & 1u) << 8;
@@ -1408,11 +1463,7 @@ namespace u26
 				}
 				if (ray_max > 0.0f)
 				{
-					// the swept edge's extent along dir (prp_compute_edge_projection_bounds with the
-					// target edges' lower bound, cached_bvh.cpp:377-473), widened by 1e-6
-					const float ep0 = dot(p0, dir), ep1 = dot(p1, dir);
-					proj_lo = fmaxf(fminf(ep0, ep1), ee_pmin - 1e-5f) - 1e-6f;
-					proj_hi = (fmaxf(ep0, ep1) + ray_max * dl2) + 1e-6f;
+					swept_extent(p0, p1, dir, dl2, ray_max, ee_pmin, proj_lo, proj_hi);
 					e1 = p1 - p0;
 					pn = cross(e1, dir);
 					const float nl = length(pn);
@@ -1422,16 +1473,7 @@ namespace u26
 						pn = pn / nl;
 						pd = dot(pn, p0);
 					}
-					const f3 a_end = p0 + dir * ray_max, b_end = p1 + dir * ray_max;
-					smn = vmin(vmin(p0, p1), vmin(a_end, b_end));
-					smx = vmax(vmax(p0, p1), vmax(a_end, b_end));
-					// intersect the swept box with the grown AABB of the candidate target edges
-					const float* tb = slot_box + 12 * size_t(ee_slot) + 6;
-					const float g0 = 1e-5f * (1.0f + fmaxf(fabsf(tb[0]), fabsf(tb[3])));
-					const float g1 = 1e-5f * (1.0f + fmaxf(fabsf(tb[1]), fabsf(tb[4])));
-					const float g2 = 1e-5f * (1.0f + fmaxf(fabsf(tb[2]), fabsf(tb[5])));
-					smn = vmax(smn, mk3(tb[0] - g0, tb[1] - g1, tb[2] - g2));
-					smx = vmin(smx, mk3(tb[3] + g0, tb[4] + g1, tb[5] + g2));
+					swept_box(p0, p1, dir, ray_max, slot_box + 12 * size_t(ee_slot) + 6, smn, smx);
 					if (smn.x <= smx.x && smn.y <= smx.y && smn.z <= smx.z)
 						kind = 2;
 				}
@@ -1448,13 +1490,10 @@ namespace u26
 				W.u[5][lane] = plane ? 1u : 0u, W.u[6][lane] = ev.x, W.u[7][lane] = ev.y;
 				__syncwarp();
 				const uint32_t tested0 = tested;
-				// Centres and half extents of the swept box and of its extent along dir. The box test below rounds
-				// them three times more than it rounds the bounds themselves, each time by at most 2^-24 of the larger
-				// bound, which the node's margin does not cover when the swept edge is some hundred times longer
-				// than the node's distance from the origin: the half extents are widened by 2^-22 of it.
-				auto half = [](float lo, float hi) { return 0.5f * (hi - lo) + 0x1p-22f * fmaxf(fabsf(lo), fabsf(hi)); };
-				const f3 sc = 0.5f * (smn + smx), sh = mk3(half(smn.x, smx.x), half(smn.y, smx.y), half(smn.z, smx.z));
-				const float proj_c = 0.5f * (proj_lo + proj_hi), proj_h = half(proj_lo, proj_hi);
+				// centres and half extents of the swept box and of its extent along dir
+				const f3 sc = 0.5f * (smn + smx);
+				const f3 sh = mk3(half_extent(smn.x, smx.x), half_extent(smn.y, smx.y), half_extent(smn.z, smx.z));
+				const float proj_c = 0.5f * (proj_lo + proj_hi), proj_h = half_extent(proj_lo, proj_hi);
 				const f3 wn = plane ? pn : mk3(0.0f); // (no plane: every box meets the slab)
 				const float wd = plane ? pd : 0.0f;
 				ray_walk(
@@ -1463,9 +1502,9 @@ namespace u26
 					// swept edge's (a box that misses it holds no edge the swept edge reaches); and it meets the
 					// slab |dot(pn, q) - pd| <= 1e-6 around the swept edge's plane (a box clear of it holds only
 					// edges the leaf's separating-plane test rejects; cached_bvh.cpp:433-473 prunes its nodes the same
-					// way). Explicit fmas: the boxes carry the 1e-5 (1 + |c|) margin, far above the rounding of
-					// the node's own terms, and the swept extents carry theirs, so no edge that the tests on
-					// the bounds themselves would keep is pruned.
+					// way). Explicit fmas; both sides' half extents carry this test's rounding (half_extent), which the
+					// 1e-5 (1 + |c|) margin of the node does not cover beside a swept edge of 1,000 units, so no edge that
+					// edge_reached keeps is pruned.
 					[&](const NodeBox& g)
 					{
 						const float cp = __fmaf_rn(g.mn.z, dir.z, __fmaf_rn(g.mn.y, dir.y, g.mn.x * dir.x));
@@ -4893,7 +4932,7 @@ static u26_status prp_run(u26_scene* S, u26_lbvh* face_tree, u26_lbvh* edge_tree
 					}
 					const RaycastFn kern = raycast_variant(rc, c.min_blocks, c.queue);
 					const LeafArgs leaf{ d_x, S->d_edges.as<uint2>(), S->d_faces.as<uint32_t>(), S->d_bits_e.as<uint32_t>(),
-						S->d_bits_f.as<uint32_t>(), es_ / 32u + 1u, fs / 32u + 1u, sink };
+						S->d_bits_f.as<uint32_t>(), es_ / 32u + 1u, fs / 32u + 1u, sink, S->d_slot_box.as<float>(), S->d_tasks.as<Task>() };
 					kern<<<uint32_t(blocks), 128, 4 * sizeof(RayWarp), st>>>(S->d_tasks.as<Task>(), nt, total_req, S->d_slots.as<Slot>(),
 						S->d_cand_v.as<uint32_t>(), S->d_cand_e.as<uint32_t>(), vs, es_, S->d_fgrow.as<NodeBox>(), S->d_egrow.as<NodeBox>(),
 						S->d_front.as<uint32_t>(), S->d_front.as<uint32_t>() + size_t(nobj) * kFrontStride, S->d_slot_box.as<float>(), leaf,
