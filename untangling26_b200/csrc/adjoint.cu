@@ -205,9 +205,10 @@ namespace u26
 			return mk3(dirs[3 * size_t(c)], dirs[3 * size_t(c) + 1], dirs[3 * size_t(c) + 2]);
 		}
 
-		// Hits that a warp takes alone: as many as one warp's rounds take no longer than a cluster's barriers (64), or, with
-		// a chip full of contours, than about two thirds of all hits' time (0.12 us a hit in one warp's chain, 55 ps of the
-		// whole chip).
+		// Hits that a warp takes alone: as many as one warp's rounds take no longer than a cluster's barriers (64; 128 where the
+		// contours' clusters take more than one wave: 148 contours of 100 hits 35 + 51 us by clusters, 23 + 37 by warps),
+		// or, with a chip full of contours, than about two thirds of all hits' time (0.12 us a hit in one warp's chain,
+		// 55 ps of the whole chip: 3,000 contours of 500 hits 103 + 251 us by blocks, 86 + 252 by warps).
 		__device__ __forceinline__ uint32_t few_hits(const uint32_t* __restrict__ off, uint32_t nc)
 		{
 			if (nc <= kManyContours)
